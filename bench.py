@@ -323,8 +323,8 @@ PERSIST_BYTES = {(2, True): (100, 48), (2, False): (68, 52),
 # variant) applies d += a p in the direction phase, reading p once.
 PERSIST_DEFER_MIN_ROWS = 3_000_000
 PERSIST_BYTES_DEFERRED = {(2, True): (96, 36)}
-PERSIST_KERNEL = {(2, True): "k_inner_persist_split<learned>", (2, False): "k_inner_persist_split<Jacobi>",
-                  (1, True): "k_inner_persist<learned>", (1, False): "k_inner_persist<Jacobi>"}
+PERSIST_KERNEL = {(2, True): "k_inner_split<learned>", (2, False): "k_inner_split<Jacobi>",
+                  (1, True): "k_inner_fused<learned>", (1, False): "k_inner_fused<Jacobi>"}
 
 
 def persist_roofline(args, results, N, peak, peak_kind):

@@ -207,9 +207,6 @@ struct cgx_handle {
   // Second buffers of the ping-pong pairs (p, r) and z of the persistent
   // inner solves (persist.cuh).
   float *p32b = nullptr, *r32b = nullptr, *z32 = nullptr;
-  // Partial sums and the barrier counter of the persistent inner solves.
-  double *persist_part = nullptr;
-  unsigned long long *persist_sync = nullptr;
   double *r64 = nullptr;
   bool f32_valid = false;
   // What the captured inner-solve graphs took from the FP32 copy (its
@@ -224,7 +221,9 @@ struct cgx_handle {
   Band band;
   bool band_tried = false;
 
-  // Scratch: state, partial sums, dot result, validation flag.
+  RedMem *red = nullptr;  // barrier state of the persistent solves (gridred.cuh)
+
+  // Scratch: state, partial sums, dot result, validation flag, barrier state.
   void *scratch = nullptr;
   CgState *st = nullptr;
   double *partials = nullptr;
@@ -389,8 +388,6 @@ static void free_matrix(cgx_handle *h) {
   h->c_valid = false;
   h->value32 = h->C32 = h->d32 = h->r32 = h->p32 = h->q32 = nullptr;
   h->p32b = h->r32b = h->z32 = nullptr;
-  h->persist_part = nullptr;
-  h->persist_sync = nullptr;
   h->r64 = nullptr;
   h->idx16 = nullptr;
   h->compact16 = false;
@@ -915,6 +912,7 @@ cgx_status cgx_create(cgx_handle **out, int device) {
   size_t o_part = c.take<double>(2 * (size_t)kMaxGrid);
   size_t o_dot = c.take<double>(4);
   size_t o_flag = c.take<int>(4);
+  size_t o_red = c.take<RedMem>(1);
   if ((e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking)) !=
           cudaSuccess ||
       (e = cudaMalloc(&h->scratch, c.off)) != cudaSuccess ||
@@ -935,6 +933,7 @@ cgx_status cgx_create(cgx_handle **out, int device) {
   h->partials = (double *)(base + o_part);
   h->dot_out = (double *)(base + o_dot);
   h->flag = (int *)(base + o_flag);
+  h->red = (RedMem *)(base + o_red);
   e = cudaMemsetAsync(h->scratch, 0, c.off, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
@@ -1816,8 +1815,6 @@ static cgx_status ensure_f32(cgx_handle *h) {
     size_t o_rb = c.take<float>((size_t)N + kPad);
     size_t o_z = c.take<float>((size_t)N + kPad);
     size_t o_r64 = c.take<double>((size_t)N + kPad);
-    size_t o_pp = c.take<double>((size_t)kPersistSlots * kMaxGrid);
-    size_t o_ps = c.take<unsigned long long>(1);
     size_t o_i16 = c.take<int16_t>((size_t)h->nz + kPad);
     CUDA_TRY(dev_alloc(h, (void **)&h->f32_mem, c.off));
     CUDA_TRY(cudaMemsetAsync(h->f32_mem, 0, c.off, h->stream));
@@ -1832,8 +1829,6 @@ static cgx_status ensure_f32(cgx_handle *h) {
     h->r32b = (float *)(base + o_rb);
     h->z32 = (float *)(base + o_z);
     h->r64 = (double *)(base + o_r64);
-    h->persist_part = (double *)(base + o_pp);
-    h->persist_sync = (unsigned long long *)(base + o_ps);
     h->idx16 = (int16_t *)(base + o_i16);
   }
   k_to_f32<<<grid_stream(h, h->nz), kThreads, 0, h->stream>>>(
@@ -1947,72 +1942,143 @@ static cudaError_t launch_learned_apply(cgx_handle *h, bool start) {
   return launch_crs_view(h, Gv, L->y32, zop);
 }
 
+// Which form an inner solve on the band takes, and the CTAs' width. Measured on
+// the 7-point grids (us per iteration):
+//              Jacobi fused / split     learned fused 256, 512 | 1024 / split
+//   24^3       4.8 / 7.3                6.6 | - / 11.3
+//   48^3       5.6 / 7.5                7.8 | 8.9 / 11.7
+//   64^3       6.8 / 8.5                10.1 | 9.9 / 13.6
+//   96^3       11.3 / 11.6              17.9 | 16.4 / 20.0
+//   112^3      14.8 / 14.3              24.8 | 21.9 / 25.5
+//   128^3      21.4 / 17.7              38.9 | 32.5 / 33.8
+// The split form prefetches the band above 3M rows (160^3: Jacobi 38.1 against
+// 40.7, learned 70.3 against 72.3; 128^3, where the band stays in L2: 19.8
+// against 18.0 and 37.6 against 35.8).
+constexpr int kInnerFusedMaxRows[2] = {1000000, 2300000};  // Jacobi, learned
+constexpr int kInnerNarrowCtaRows = 148 * 256;  // 256-thread CTAs up to here
+constexpr int kInnerWideCtaRows = 200000;       // learned: 1024 from here on
+constexpr int kInnerPrefetchMinRows = 3000000;
+// SELL-U: 512-thread CTAs up to two passes of them, 1024 beyond (27-point grids,
+// Jacobi / learned: 24^3 9.2 / 15.7 against 11.9 / 20.8 us per iteration, 48^3
+// 10.0 / 20.2 against 12.4 / 23.3, 64^3 15.2 / 30.6 against 13.8 / 25.0, 96^3
+// 32.1 / 69.8 against 27.0 / 51.9).
+constexpr int kInnerSellNarrowRows = 148 * 1024;
+
 // One inner solve as a persistent cooperative launch (persist.cuh), after
-// the path's start kernel(s). The grid is what the SMs hold at once, as a
-// cooperative launch requires (and no more CTAs than 256-row tiles or
-// partial-sum slots).
+// the path's start kernel(s): one CTA per SM, and no more CTAs than tiles.
 enum class InnerForm { kGraph, kFused, kSplit, kSell };
 
-static cudaError_t launch_inner_persist(cgx_handle *h, bool learned, InnerForm form) {
-  PersistArgs a;
-  a.p[0] = h->p32;
-  a.p[1] = h->p32b;
-  a.r[0] = h->r32;
-  a.r[1] = h->r32b;
-  a.z = learned ? h->L->z32 : h->z32;
+// A cooperative launch over `grid` CTAs of T threads with room for `smem` bytes
+// of resident vectors.
+static cudaError_t launch_coop(cgx_handle *h, const void *kern, int grid, int T, size_t smem,
+                               void **args) {
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->red, 0, kRedZeroBytes, h->stream);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchCooperativeKernel(kern, grid, T, args, smem, h->stream);
+}
+
+template <typename Phases, int T>
+static cudaError_t launch_inner_split(cgx_handle *h, const Phases &P, InnerArgs a) {
+  const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+  a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
+  int room = kInnerResident / (int)(T * sizeof(float));
+  auto take = [&](bool wanted) {
+    const int n = wanted ? std::min(room, a.steps) : 0;
+    room -= n;
+    return n;
+  };
+  // Bytes a row and iteration that 4 resident bytes save: Jacobi r 12, d, q
+  // and C 8; learned z, d, q and the copy of r 8.
+  if (Phases::kLearned) {
+    a.nz = take(Phases::kTiled);
+    a.nd = take(true);
+    a.nq = take(Phases::kTiled);
+    a.nr = take(Phases::kTiled);
+  } else {
+    a.nr = take(true);
+    a.nd = take(true);
+    a.nq = take(Phases::kTiled);
+    a.nc = take(true);
+  }
+  const size_t smem = sizeof(float) * T * (size_t)(a.nz + a.nr + a.nd + a.nq + a.nc);
+  CgState *st = h->st;
+  void *args[] = {(void *)&P, &a, &st};
+  return launch_coop(h, (const void *)k_inner_split<Phases, T>, grid, T, smem, args);
+}
+
+template <bool LEARNED, int T>
+static cudaError_t launch_inner_fused(cgx_handle *h, BandView<4> A, GBandView G, InnerArgs a) {
+  int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+  a.rows = (int)round_up((size_t)((h->N + grid - 1) / grid), 32);
+  grid = (h->N + a.rows - 1) / a.rows;
+  a.steps = (a.rows + T - 1) / T;
+  // Offsets ascend, with 0 in the padding slots.
+  const int reach = *std::max_element(A.d, A.d + 4);
+  if (LEARNED) a.below = std::min(grid, (reach + a.rows - 1) / a.rows);
+  int room = kInnerResident / (int)(T * sizeof(float));
+  auto take = [&](bool wanted) {
+    const int n = wanted ? std::min(room, a.steps) : 0;
+    room -= n;
+    return n;
+  };
+  a.nr = take(!LEARNED);
+  a.nd = take(true);
+  a.nq = take(!LEARNED);
+  a.nc = take(true);
+  const size_t smem = sizeof(float) * T * (size_t)(a.nr + a.nd + a.nq + a.nc);
+  CgState *st = h->st;
+  void *args[] = {&A, &G, &a, &st};
+  return launch_coop(h, (const void *)k_inner_fused<LEARNED, T>, grid, T, smem, args);
+}
+
+template <bool LEARNED>
+static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
+  InnerArgs a{};
+  a.p = h->p32;
+  a.p2 = h->p32b;
+  a.r = h->r32;
+  a.r2 = h->r32b;
+  a.z = LEARNED ? h->L->z32 : h->z32;
   a.d = h->d32;
   a.q = h->q32;
-  a.y = learned ? h->L->y32 : nullptr;
+  a.y = LEARNED ? h->L->y32 : nullptr;
   a.C = h->C32;
-  a.eps = learned ? h->L->eps : 0.f;
-  a.part = h->persist_part;
-  a.sync = h->persist_sync;
-  CgState *st = h->st;
-  // The grid: as many CTAs as the SMs hold, at most one per T-row tile.
-  auto grid_for = [&](const void *kern, int T, int *grid) {
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, 0);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorCooperativeLaunchTooLarge;
-    const long long tiles = ((long long)h->N + T - 1) / T;
-    *grid = (int)std::max<long long>(
-        1, std::min<long long>({(long long)h->num_sms * per_sm, kMaxGrid, tiles}));
-    return cudaMemsetAsync(a.sync, 0, sizeof(unsigned long long), h->stream);
-  };
-  int grid = 0;
-  cudaError_t e;
+  a.eps = LEARNED ? h->L->eps : 0.f;
+  a.red = h->red;
   if (form == InnerForm::kSell) {
-    constexpr int T = kPersistSellThreads, B = kPersistSellMinB;
     const SellUView<float> A{h->sa.meta, h->sa.off, h->sa_val, h->N};
     SellUView<__nv_bfloat16> G{}, GT{};
-    if (learned) {
+    if (LEARNED) {
       G = SellUView<__nv_bfloat16>{h->L->sg.meta, h->L->sg.off, h->L->sg_val, h->N};
       GT = SellUView<__nv_bfloat16>{h->L->st.meta, h->L->st.off, h->L->st_val, h->N};
     }
-    const void *kern = learned ? (const void *)k_inner_persist_sell<true, T, B>
-                               : (const void *)k_inner_persist_sell<false, T, B>;
-    if ((e = grid_for(kern, T, &grid)) != cudaSuccess) return e;
-    void *args[] = {(void *)&A, &G, &GT, &a, &st};
-    return cudaLaunchCooperativeKernel(kern, grid, T, args, 0, h->stream);
+    if (h->N <= kInnerSellNarrowRows)
+      return launch_inner_split<SellPhases<LEARNED, 512>, 512>(
+          h, SellPhases<LEARNED, 512>{A, G, GT}, a);
+    return launch_inner_split<SellPhases<LEARNED, 1024>, 1024>(
+        h, SellPhases<LEARNED, 1024>{A, G, GT}, a);
   }
-  BandView<4> A = band_view(h);
+  const BandView<4> A = band_view(h);
   GBandView G{};
-  if (learned) G = gband_view(h);
-  constexpr int T = kPersistThreads, F = kPersistFusedMinB;
-  constexpr int SL = kPersistSplitMinB[1], SJ = kPersistSplitMinB[0];
-  constexpr int PF = kPersistPrefetchRows;
-  const bool split = form == InnerForm::kSplit;
-  const bool pf = h->N >= kPersistPrefetchMinRows;
-  const void *kern =
-      split ? (learned ? (pf ? (const void *)k_inner_persist_split<true, T, SL, PF>
-                             : (const void *)k_inner_persist_split<true, T, SL, 0>)
-                       : (pf ? (const void *)k_inner_persist_split<false, T, SJ, PF>
-                             : (const void *)k_inner_persist_split<false, T, SJ, 0>))
-            : (learned ? (const void *)k_inner_persist<true, T, F>
-                       : (const void *)k_inner_persist<false, T, F>);
-  if ((e = grid_for(kern, T, &grid)) != cudaSuccess) return e;
-  void *args[] = {&A, &G, &a, &st};
-  return cudaLaunchCooperativeKernel(kern, grid, T, args, 0, h->stream);
+  if (LEARNED) G = gband_view(h);
+  if (form == InnerForm::kFused) {
+    if (h->N <= kInnerNarrowCtaRows) return launch_inner_fused<LEARNED, 256>(h, A, G, a);
+    if (LEARNED && h->N >= kInnerWideCtaRows)
+      return launch_inner_fused<LEARNED, 1024>(h, A, G, a);
+    return launch_inner_fused<LEARNED, 512>(h, A, G, a);
+  }
+  constexpr int T = 1024;
+  if (h->N >= kInnerPrefetchMinRows)
+    return launch_inner_split<BandPhases<LEARNED, true, T>, T>(
+        h, BandPhases<LEARNED, true, T>{A, G}, a);
+  return launch_inner_split<BandPhases<LEARNED, false, T>, T>(
+      h, BandPhases<LEARNED, false, T>{A, G}, a);
+}
+
+static cudaError_t launch_inner_persist(cgx_handle *h, bool learned, InnerForm form) {
+  return learned ? launch_inner_persist<true>(h, form) : launch_inner_persist<false>(h, form);
 }
 
 // The SELL-U form of the persistent inner solve needs A's inner product on
@@ -2041,7 +2107,7 @@ static bool persist_fits(const cgx_handle *h, bool learned) {
 
 // Which inner solve a mixed solve runs: the graph of per-iteration kernels,
 // or a persistent launch per inner solve, fused (systems up to
-// kPersistFusedMaxRows rows) or split (larger ones). CGX_LOOP_PERSISTENT and
+// kInnerFusedMaxRows rows) or split (larger ones). CGX_LOOP_PERSISTENT and
 // CGX_LOOP_PERSISTENT_SPLIT force their form on the band; the default
 // CGX_LOOP_GRAPH takes the persistent form that measured fastest.
 static InnerForm inner_form(const cgx_handle *h, const cgx_options &o, bool learned) {
@@ -2052,7 +2118,7 @@ static InnerForm inner_form(const cgx_handle *h, const cgx_options &o, bool lear
   if (o.loop == CGX_LOOP_PERSISTENT) return InnerForm::kFused;
   if (o.loop == CGX_LOOP_PERSISTENT_SPLIT) return InnerForm::kSplit;
   if (o.loop != CGX_LOOP_GRAPH) return InnerForm::kGraph;
-  return h->N <= kPersistFusedMaxRows ? InnerForm::kFused : InnerForm::kSplit;
+  return h->N <= kInnerFusedMaxRows[learned] ? InnerForm::kFused : InnerForm::kSplit;
 }
 
 static cudaError_t launch_learned_start(cgx_handle *h) {
@@ -2109,28 +2175,18 @@ static cgx_status solve_mixed(cgx_handle *h, const cgx_options &o,
   CUDA_TRY(cudaEventRecord(h->ev[6], s));
   CGX_TRY(ensure_f32(h));
 
-  // The persistent inner solves (persist.cuh): the fused form, and the split
-  // one where persist_defers_d, leave d's last update pending; the fused
-  // form's start also stores z.
+  // The persistent inner solves (persist.cuh); the fused form's start also
+  // stores z.
   const InnerForm form = inner_form(h, o, want_learned);
   const bool persist = form != InnerForm::kGraph;
-  const bool pending =
-      form == InnerForm::kFused ||
-      (form == InnerForm::kSplit &&
-       persist_defers_d(want_learned,
-                        h->N >= kPersistPrefetchMinRows ? kPersistPrefetchRows : 0));
   // PERSISTENT on a matrix without the band form runs as GRAPH.
   const bool graph_loop =
       (o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT ||
        o.loop == CGX_LOOP_PERSISTENT_SPLIT) &&
       !persist;
   auto outer_update = [&] {
-    if (pending)
-      k_outer_update_pending<<<grid_stream(h, h->N), kThreads, 0, h->stream>>>(
-          h->N, h->vec[CGX_VECTOR_X], h->d32, h->p32, h->p32b, h->st);
-    else
-      k_outer_update<<<grid_stream(h, h->N), kThreads, 0, h->stream>>>(
-          h->N, h->vec[CGX_VECTOR_X], h->d32, h->st);
+    k_outer_update<<<grid_stream(h, h->N), kThreads, 0, h->stream>>>(
+        h->N, h->vec[CGX_VECTOR_X], h->d32, h->st);
     return cudaGetLastError();
   };
   auto guard = [&] {
@@ -3166,9 +3222,9 @@ cgx_status cgx_check_wait_timeout(cgx_handle *h, int which, int *error_bits) {
   CGX_TRY(ensure_f32(h));
   reset_host_state(h, 1, 0.0, false, 0);
   CGX_TRY(push_state(h));
-  CUDA_TRY(cudaMemsetAsync(h->persist_sync, 0, sizeof(unsigned long long), h->stream));
+  CUDA_TRY(cudaMemsetAsync(h->red, 0, kRedZeroBytes, h->stream));
   // Two CTAs, 4096 polls each: a few milliseconds before they give up.
-  k_wait_timeout<<<2, 128, 0, h->stream>>>(h->persist_sync, which, 4096u, h->st);
+  k_wait_timeout<<<2, 128, 0, h->stream>>>(h->red, which, 4096u, h->st);
   CUDA_TRY(cudaGetLastError());
   CGX_TRY(pull_state(h));
   *error_bits = h->host_st->error;

@@ -41,7 +41,6 @@ struct CgState {
   double inner_tol_min;  // floor of the inner relative tolerance
   int in_iter, in_stop, in_finished;
   int total_inner;
-  int in_pslot;  // fused persistent inner solve: ping-pong buffer of the last p
 };
 
 // The inner FP32 iteration cannot make progress: a step length that is zero
@@ -53,6 +52,12 @@ __device__ __forceinline__ bool inner_broke_down(const CgState *st) {
   const double a = st->in_alpha;
   return !(fabs(a) <= 1.7976931348623157e308) || a == 0.0;
 }
+
+// A compile-time number as a function argument.
+template <int V>
+struct IntTag {
+  static constexpr int value = V;
+};
 
 // --- reductions ------------------------------------------------------------
 

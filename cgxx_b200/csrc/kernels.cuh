@@ -1095,20 +1095,4 @@ __global__ void __launch_bounds__(kThreads)
     x[i] = fma(s, (double)d[i], x[i]);
 }
 
-// The same after a fused band inner solve, whose last update of d is still
-// pending: x += ||r64|| (d + a p), with p the buffer of the pair that the
-// last iteration wrote and d + a p rounded as the unfused update rounds it.
-__global__ void __launch_bounds__(kThreads)
-    k_outer_update_pending(int N, double *__restrict__ x,
-                           const float *__restrict__ d,
-                           const float *__restrict__ p0,
-                           const float *__restrict__ p1, const CgState *st) {
-  const double s = sqrt(st->r2);
-  const float a = (float)st->in_alpha;
-  const float *__restrict__ p = st->in_pslot ? p1 : p0;
-  for (int i = blockIdx.x * kThreads + threadIdx.x; i < N;
-       i += gridDim.x * kThreads)
-    x[i] = fma(s, (double)fmaf(a, p[i], d[i]), x[i]);
-}
-
 }  // namespace cgx
