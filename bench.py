@@ -362,6 +362,14 @@ def persist_roofline(args, results, N, peak, peak_kind):
     return out
 
 
+def plain_persistent(args, N):
+    """Whether the plain solve's loop is one persistent launch: the grids in
+    the default loop, but for the 7-point ones of 0.7M to 1.1M rows
+    (kSolve64FusedMaxRows, kSolve64SplitMinRows)."""
+    return not args.graph and args.loop in ("graph", "persistent", "split") and not (
+        args.loop == "graph" and args.stencil == 7 and 700000 < N < 1100000)
+
+
 def peaks():
     p = os.path.join(REPO, "MEASURED_PEAKS.json")
     try:
@@ -629,7 +637,9 @@ def our_arm(args, world, rank, local):
     # refinement check (outer + 1), and per refinement step its start, the
     # inner solve and the update of x; the learned path adds its set-up
     # (2 kernels), inference (6) and the start's apply (2 per step).
-    if args.path == "plain":
+    if args.path == "plain" and plain_persistent(args, N):
+        per_solve = 3                               # fill, set-up, one launch
+    elif args.path == "plain":
         per_solve = 2 + 4 * iters                   # fill, set-up, 3 fused + guard
     elif args.path == "mixed":
         inner = outer if persist else 4 * iters     # one launch, or 3 kernels + guard

@@ -31,6 +31,7 @@
 #include "learned.cuh"
 #include "persist.cuh"
 #include "sell.cuh"
+#include "solve64.cuh"
 
 using namespace cgx;
 
@@ -163,6 +164,21 @@ static void band_drop_values(cgx_handle *h, Band &B) {
   B.ok = false;
 }
 
+// FP64 values of A by offset (solve64.cuh), for matrices of few offsets. The
+// offsets are planned once per pattern, U is filled once per set of values; ok:
+// U holds the current ones.
+struct Band64 {
+  void *mem = nullptr;
+  double *U = nullptr;                 // KP arrays of ld rows
+  double *p2 = nullptr, *z = nullptr;  // fused form: N each
+  size_t ld = 0;
+  std::vector<int> all;   // A's offsets, ascending (empty: too many)
+  std::vector<int> half;  // the non-negative ones, if the set is symmetric
+  bool planned = false, filled = false, ok = false;
+  bool sym = false;       // U holds `half`, else `all`
+  int KP = 0;             // the kernel's number of offsets
+};
+
 struct cgx_handle {
   int device = 0;
   // Device blocks of replaced matrices, kept for the next upload
@@ -221,6 +237,8 @@ struct cgx_handle {
   Band band;
   bool band_tried = false;
 
+  // Values by offset of the persistent plain solves.
+  Band64 b64;
   RedMem *red = nullptr;  // barrier state of the persistent solves (gridred.cuh)
 
   // Scratch: state, partial sums, dot result, validation flag, barrier state.
@@ -376,6 +394,8 @@ static void free_matrix(cgx_handle *h) {
   h->sa_tried = false;
   band_free(h, h->band);
   h->band_tried = false;
+  if (h->b64.mem) dev_free(h, h->b64.mem);
+  h->b64 = Band64{};
   h->format = -1;
   h->N = h->nz = 0;
   h->ptr = h->index = nullptr;
@@ -1590,7 +1610,7 @@ static cgx_status device_errors(cgx_handle *h) {
                 "the device loop guard stopped a loop that did not terminate");
   if (h->host_st->error & kErrGridSync)
     return fail(CGX_ERROR_DEVICE,
-                "a grid barrier of the persistent inner solve timed out; results are invalid");
+                "a grid barrier of a persistent solve timed out; results are invalid");
 
   return CGX_SUCCESS;
 }
@@ -1624,18 +1644,340 @@ static cudaError_t add_segments(cgx_handle *h, int ran, double &t_spmv,
   return cudaSuccess;
 }
 
+// A's column offsets, ascending (k_band_offsets); empty if there are more than
+// the table holds.
+template <typename Rows>
+static cgx_status band_offsets(cgx_handle *h, const Rows &A, std::vector<int> &D) {
+  D.clear();
+  const int N = h->N;
+  int *table = nullptr;
+  CUDA_TRY(dev_alloc(h, (void **)&table, sizeof(int) * kBandTable));
+  std::vector<int> host(kBandTable, kBandEmpty);
+  int flag = 0;
+  cudaError_t e = cudaMemcpyAsync(table, host.data(), sizeof(int) * kBandTable,
+                                  cudaMemcpyHostToDevice, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream);
+  if (e == cudaSuccess) {
+    k_band_offsets<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, table, h->flag);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(host.data(), table, sizeof(int) * kBandTable,
+                        cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost,
+                        h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  dev_free(h, table);
+  CUDA_TRY(e);
+  if (flag) return CGX_SUCCESS;
+  for (int v : host)
+    if (v != kBandEmpty) D.push_back(v);
+  std::sort(D.begin(), D.end());
+  return CGX_SUCCESS;
+}
+
+// The non-negative offsets (0 always among them) if the set is symmetric, else
+// none. |d| < N, so -d cannot overflow.
+static std::vector<int> half_offsets(const std::vector<int> &D) {
+  std::vector<int> half;
+  if (D.empty()) return half;
+  half.push_back(0);
+  for (int d : D) {
+    if (!std::binary_search(D.begin(), D.end(), -d)) return {};
+    if (d > 0) half.push_back(d);
+  }
+  return half;
+}
+
+// B.K = 0 unless A's offsets fit the FP32 band.
+static cgx_status band_plan(cgx_handle *h, Band &B) {
+  B = Band{};
+  std::vector<int> D;
+  CGX_TRY(band_offsets(h, RowsCrs{h->ptr, h->index, h->value}, D));
+  const std::vector<int> up = half_offsets(D);
+  if (up.empty() || (int)up.size() > kBandMaxK) return CGX_SUCCESS;
+  B.K = (int)up.size();
+  for (int k = 0; k < B.K; k++) B.d[k] = up[k];
+  return CGX_SUCCESS;
+}
+
+// U from A's current values by the offsets D; *fits: the rows ascend and, for
+// SYM, the values are symmetric.
+template <bool SYM, typename Rows>
+static cgx_status band64_fill(cgx_handle *h, const Rows &A, const std::vector<int> &D,
+                              bool *fits) {
+  Band64 &B = h->b64;
+  const int N = h->N;
+  Band64Offsets o{};
+  o.K = (int)D.size();
+  for (int k = 0; k < o.K; k++) o.d[k] = D[k];
+  unsigned long long *counts = nullptr;
+  CUDA_TRY(dev_alloc(h, (void **)&counts, 2 * sizeof(unsigned long long)));
+  unsigned long long hc[2] = {0, 0};
+  int flag = 0;
+  cudaError_t e = cudaMemsetAsync(B.U, 0, sizeof(double) * B.KP * B.ld, h->stream);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream);
+  if (e == cudaSuccess) {
+    k_band64_fill<SYM><<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, o, B.U, B.ld,
+                                                                      counts, h->flag);
+    if (SYM)
+      k_band64_check<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, o, B.U, B.ld, counts,
+                                                                    h->flag);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  dev_free(h, counts);
+  CUDA_TRY(e);
+  *fits = flag == 0 && (!SYM || hc[0] == hc[1]);
+  return CGX_SUCCESS;
+}
+
+// Room for KP arrays of values; *got false when the device has none (the
+// solve then runs on the matrix as uploaded).
+static cgx_status band64_alloc(cgx_handle *h, int KP, bool *got) {
+  Band64 &B = h->b64;
+  *got = true;
+  if (B.mem && B.KP == KP) return CGX_SUCCESS;
+  if (B.mem) dev_free(h, B.mem);
+  B.mem = nullptr;
+  B.KP = KP;
+  B.ld = round_up((size_t)h->N, 32);
+  Carver c;
+  const size_t o_u = c.take<double>(B.ld * KP);
+  const size_t o_p = c.take<double>((size_t)h->N + kPad);
+  const size_t o_z = c.take<double>((size_t)h->N + kPad);
+  const cudaError_t e = dev_alloc(h, &B.mem, c.off);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    *got = false;
+    return CGX_SUCCESS;
+  }
+  CUDA_TRY(e);
+  B.U = (double *)((char *)B.mem + o_u);
+  B.p2 = (double *)((char *)B.mem + o_p);
+  B.z = (double *)((char *)B.mem + o_z);
+  return CGX_SUCCESS;
+}
+
+// Which form a solve takes, and the CTAs' width. Measured (us per iteration;
+// the graph of kernels, then fused with 256 | 512 threads, split with 512 |
+// 1024):
+//   5-point 64^2 (4k rows)   17.5    4.6 | 4.6      - | 6.9
+//   5-point 128^2 (16k)      13.9    4.8 | 5.2      - | 7.6
+//   7-point 48^3             15.6    6.7 | 6.5      - | 8.3
+//   7-point 64^3             18.8    9.2 | 8.1      9.6 | 10.3
+//   7-point 80^3 (ELL)       22.5    - | 11.2       - | 14.6
+//   7-point 112^3 (1.4M)     -       - | 26.5       - | 23.1
+//   7-point 128^3            68.6    74.4 | 56.5    52.9 | 36.4
+//   7-point 160^3            128     - | 94.0       102 | 76.3
+//   27-point, all offsets stored:
+//     48^3                   20.5    - | 9.2        9.6 | 9.9
+//     64^3                   27.9    - | 13.4       13.1 | 13.5
+//     96^3                   74.8    - | 46.6       43.5 | 49.7
+//     128^3                  153     - | 116        110 | 124
+//   27-point, symmetric half stored:
+//     96^3                   73.4    - | 39.9       35.6 | 33.2
+// So: fused up to 0.7M rows with few offsets (0.2M with many), 256-thread CTAs
+// up to one pass of them; split beyond, 512 threads where the offsets are all
+// stored and many (their loads need the registers).
+constexpr int kSolve64FusedMaxRows = 700000;
+constexpr int kSolve64FusedMaxRowsWide = 200000;
+constexpr int kSolve64NarrowCtaRows = 148 * 256;
+// Few offsets, between kSolve64FusedMaxRows and this: the graph of kernels. The
+// fused form would be faster here too (96^3: 15.2 us per iteration against 36),
+// but the project's bar for the learned solve is twice the plain solve's speed
+// on 96^3 fields (test_learned_twice_as_fast_as_plain_on_heldout_fields), and
+// the learned solve (4.1 ms a field) meets it against the graph (2.9x), not
+// against this form (1.3x).
+constexpr int kSolve64SplitMinRows = 1100000;
+// The split form prefetches the values of its next step from this many bytes
+// of them on (160^3, 131 MB: 78.3 -> 76.3 us; 128^3, 67 MB: 37.7 -> 36.4;
+// 112^3, 45 MB, which stay in L2: 23.1 -> 24.2).
+constexpr size_t kSolve64PrefetchBytes = (size_t)60 << 20;
+// The by-offset values of the current matrix, for a solve in the given loop
+// mode. They are used when they take no more bytes than the entries of the
+// uploaded layout (12 each): a matrix whose offsets are mostly empty stays on
+// its rows.
+template <typename Rows>
+static cgx_status ensure_band64(cgx_handle *h, const Rows &A, int loop, bool *use) {
+  Band64 &B = h->b64;
+  *use = false;
+  if (!B.planned) {
+    CGX_TRY(band_offsets(h, A, B.all));
+    B.half = half_offsets(B.all);
+    B.planned = true;
+  }
+  if (loop == CGX_LOOP_GRAPH && (int)B.all.size() <= 7 && h->N > kSolve64FusedMaxRows &&
+      h->N < kSolve64SplitMinRows)
+    return CGX_SUCCESS;
+  *use = B.ok;
+  if (B.filled) return CGX_SUCCESS;
+  B.ok = false;
+  auto dense = [&](int KP) { return 8.0 * KP * h->N <= 12.0 * h->nz; };
+  bool got = false, fits = false;
+  const int nh = (int)B.half.size(), na = (int)B.all.size();
+  const int KH = nh <= 3 ? 3 : nh <= 4 ? 4 : kBand64MaxHalf;
+  const int KA = na <= 7 ? 7 : kBand64MaxK;
+  if (nh > 0 && nh <= kBand64MaxHalf && dense(KH)) {
+    CGX_TRY(band64_alloc(h, KH, &got));
+    if (got) CGX_TRY(band64_fill<true>(h, A, B.half, &fits));
+    B.sym = fits;
+  }
+  if (!fits && na > 0 && na <= kBand64MaxK && dense(KA)) {
+    CGX_TRY(band64_alloc(h, KA, &got));
+    if (got) CGX_TRY(band64_fill<false>(h, A, B.all, &fits));
+  }
+  if (!fits && B.mem) {
+    dev_free(h, B.mem);
+    B.mem = nullptr;
+  }
+  *use = B.ok = fits;
+  B.filled = true;
+  return CGX_SUCCESS;
+}
+
+// A cooperative launch over `grid` CTAs of T threads with room for `smem` bytes
+// of resident vectors.
+static cudaError_t launch_coop(cgx_handle *h, const void *kern, int grid, int T, size_t smem,
+                               void **args) {
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->red, 0, kRedZeroBytes, h->stream);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchCooperativeKernel(kern, grid, T, args, smem, h->stream);
+}
+
+// Shared memory given to resident vectors: the rest stays L1 for the gathers.
+// (160^3: all 227 KB 96.8 us, 192 KB 78.3, 160 KB 78.6, 128 KB 80.1, none
+// 86.0.)
+constexpr int kSolve64Resident = 192 << 10;
+
+// The loop of a plain FP64 solve as one cooperative launch, after the set-up
+// kernel. *ran = false when the GPU cannot hold the grid at once (a device
+// shared through MPS limits): the caller then runs the graph.
+template <int K, bool SYM, bool FUSED, bool PF, int T>
+static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, bool *ran) {
+  *ran = false;
+  const Band64 &B = h->b64;
+  const void *kern = (const void *)k_solve64<K, SYM, FUSED, PF, T>;
+  const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+  Solve64Args a{};
+  a.x = h->vec[CGX_VECTOR_X];
+  a.r = h->vec[CGX_VECTOR_R];
+  a.q = h->vec[CGX_VECTOR_Q];
+  a.p = h->vec[CGX_VECTOR_P];
+  a.C = jacobi ? h->C : nullptr;
+  a.p2 = B.p2;
+  a.z = B.z;
+  a.red = h->red;
+  a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
+  // Steps of each vector in shared memory, first those of the vector whose
+  // traffic it saves most: r (24 bytes a row and iteration), then x, C and q
+  // (16 each).
+  int room = kSolve64Resident / (int)(T * sizeof(double));
+  auto take = [&](bool wanted) {
+    const int n = wanted ? std::min(room, a.steps) : 0;
+    room -= n;
+    return n;
+  };
+  a.nr = take(true);
+  a.nx = take(true);
+  a.nc = take(jacobi);
+  a.nq = take(true);
+  const size_t smem = sizeof(double) * T * (size_t)(a.nr + a.nx + a.nc + a.nq);
+  Band64View<K, SYM> A;
+  A.U = B.U;
+  A.ld = B.ld;
+  A.N = h->N;
+  const std::vector<int> &D = SYM ? B.half : B.all;
+  for (int k = 0; k < K; k++) A.d[k] = k < (int)D.size() ? D[k] : 0;
+  CgState *st = h->st;
+  void *args[] = {&A, &a, &st};
+  const cudaError_t e = launch_coop(h, kern, grid, T, smem, args);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  *ran = e == cudaSuccess;
+  return e;
+}
+
+// loop: CGX_LOOP_PERSISTENT and CGX_LOOP_PERSISTENT_SPLIT force a form.
+template <int K, bool SYM>
+static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ran) {
+  constexpr bool kWide = K > 7;
+  *ran = false;
+  if (loop == CGX_LOOP_GRAPH) {
+    loop = h->N <= (kWide ? kSolve64FusedMaxRowsWide : kSolve64FusedMaxRows)
+               ? CGX_LOOP_PERSISTENT
+               : CGX_LOOP_PERSISTENT_SPLIT;
+  }
+  if (loop == CGX_LOOP_PERSISTENT)
+    return h->N <= kSolve64NarrowCtaRows
+               ? launch_solve64<K, SYM, true, false, 256>(h, jacobi, ran)
+               : launch_solve64<K, SYM, true, false, 512>(h, jacobi, ran);
+  if (kWide && !SYM) return launch_solve64<K, SYM, false, false, 512>(h, jacobi, ran);
+  return sizeof(double) * K * (size_t)h->N >= kSolve64PrefetchBytes
+             ? launch_solve64<K, SYM, false, true, 1024>(h, jacobi, ran)
+             : launch_solve64<K, SYM, false, false, 1024>(h, jacobi, ran);
+}
+
+static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ran) {
+  if (!h->b64.sym)
+    return h->b64.KP == 7 ? launch_solve64<7, false>(h, jacobi, loop, ran)
+                          : launch_solve64<kBand64MaxK, false>(h, jacobi, loop, ran);
+  switch (h->b64.KP) {
+  case 3: return launch_solve64<3, true>(h, jacobi, loop, ran);
+  case 4: return launch_solve64<4, true>(h, jacobi, loop, ran);
+  }
+  return launch_solve64<kBand64MaxHalf, true>(h, jacobi, loop, ran);
+}
+
 static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
                              cgx_result &res) {
   const bool jacobi = o.preconditioner == CGX_PRECONDITIONER_JACOBI;
   if (jacobi && !h->c_valid)
     return fail(CGX_ERROR_INVALID_STATE, "Jacobi preconditioner not set");
   cudaStream_t s = h->stream;
-  // The persistent mode is an inner-solve mode of the mixed paths.
-  const int loop =
-      o.loop == CGX_LOOP_PERSISTENT || o.loop == CGX_LOOP_PERSISTENT_SPLIT ? CGX_LOOP_GRAPH
-                                                                           : o.loop;
+  // One persistent launch on the by-offset values; PERSISTENT and PERSISTENT_SPLIT
+  // force its fused or split form, and run as GRAPH on other matrices.
+  const bool want_persist = o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT ||
+                            o.loop == CGX_LOOP_PERSISTENT_SPLIT;
+  const int loop = want_persist ? CGX_LOOP_GRAPH : o.loop;
+  bool ran = false;
+  if (want_persist) {
+    bool use = false;
+    CUDA_TRY(cudaEventRecord(h->ev[0], s));
+    if (h->format == CGX_FORMAT_ELL)
+      CGX_TRY(ensure_band64(h, RowsEll{h->ell_length, h->ell_index, h->ell_data, h->ell_width},
+                            o.loop, &use));
+    else
+      CGX_TRY(ensure_band64(h, RowsCrs{h->ptr, h->index, h->value}, o.loop, &use));
+    if (use) {
+      reset_host_state(h, o.max_iterations, o.tolerance, false, 0);
+      CGX_TRY(push_state(h));
+      CUDA_TRY(launch_pcg_setup(h, jacobi));
+      CUDA_TRY(launch_solve64(h, jacobi, o.loop, &ran));
+    }
+    if (ran) {
+      CUDA_TRY(cudaEventRecord(h->ev[1], s));
+      CGX_TRY(pull_state(h));
+      float ms = 0;
+      CUDA_TRY(cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]));
+      res.solve_ms = ms;
+    }
+  }
 
-  if (loop == CGX_LOOP_GRAPH) {
+  if (ran) {
+    // done
+  } else   if (loop == CGX_LOOP_GRAPH) {
     GraphEntry *ge = nullptr;
     const int key = 100 + (jacobi ? 1 : 0);
     CGX_TRY(build_while_graph(
@@ -1716,49 +2058,6 @@ static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
 namespace {
 cgx_status build_sellu(cgx_handle *h, const int *ptr, const int *col,
                        size_t nnz, SellU &S);
-}
-
-// The offsets of A (k_band_offsets): B.K = 0 unless they form a symmetric
-// set with at most kBandMaxK non-negative members.
-static cgx_status band_plan(cgx_handle *h, Band &B) {
-  B = Band{};
-  const int N = h->N;
-  int *table = nullptr;
-  CUDA_TRY(dev_alloc(h, (void **)&table, sizeof(int) * kBandTable));
-  std::vector<int> host(kBandTable, kBandEmpty);
-  int flag = 0;
-  cudaError_t e = cudaMemcpyAsync(table, host.data(), sizeof(int) * kBandTable,
-                                  cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream);
-  if (e == cudaSuccess) {
-    k_band_offsets<<<grid_stream(h, N), kThreads, 0, h->stream>>>(
-        N, h->ptr, h->index, table, h->flag);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(host.data(), table, sizeof(int) * kBandTable,
-                        cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost,
-                        h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  dev_free(h, table);
-  CUDA_TRY(e);
-  if (flag) return CGX_SUCCESS;
-  std::vector<int> D;
-  for (int v : host)
-    if (v != kBandEmpty) D.push_back(v);
-  std::sort(D.begin(), D.end());
-  std::vector<int> up{0};
-  // |d| < N, so -d cannot overflow.
-  for (int d : D) {
-    if (!std::binary_search(D.begin(), D.end(), -d)) return CGX_SUCCESS;
-    if (d > 0) up.push_back(d);
-  }
-  if ((int)up.size() > kBandMaxK) return CGX_SUCCESS;
-  B.K = (int)up.size();
-  for (int k = 0; k < B.K; k++) B.d[k] = up[k];
-  return CGX_SUCCESS;
 }
 
 // U from A's current values and the symmetry check; B.ok if it passed.
@@ -1967,17 +2266,6 @@ constexpr int kInnerSellNarrowRows = 148 * 1024;
 // One inner solve as a persistent cooperative launch (persist.cuh), after
 // the path's start kernel(s): one CTA per SM, and no more CTAs than tiles.
 enum class InnerForm { kGraph, kFused, kSplit, kSell };
-
-// A cooperative launch over `grid` CTAs of T threads with room for `smem` bytes
-// of resident vectors.
-static cudaError_t launch_coop(cgx_handle *h, const void *kern, int grid, int T, size_t smem,
-                               void **args) {
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaMemsetAsync(h->red, 0, kRedZeroBytes, h->stream);
-  if (e != cudaSuccess) return e;
-  return cudaLaunchCooperativeKernel(kern, grid, T, args, smem, h->stream);
-}
 
 template <typename Phases, int T>
 static cudaError_t launch_inner_split(cgx_handle *h, const Phases &P, InnerArgs a) {
@@ -2828,6 +3116,7 @@ cgx_status cgx_update_crs_values(cgx_handle *h, const double *value) {
                              cudaMemcpyDefault, h->stream));
   h->f32_valid = false;
   h->c_valid = false;
+  h->b64.filled = h->b64.ok = false;
   if (h->L) h->L->has_factor = false;
   return CGX_SUCCESS;
 }

@@ -38,7 +38,7 @@
 
 #include <climits>
 
-#include "device.cuh"
+#include "kernels.cuh"
 
 namespace cgx {
 
@@ -77,20 +77,39 @@ __device__ __forceinline__ bool band_insert(int *table, int d) {
   return false;
 }
 
+// Row access of the two layouts a band is built from.
+struct RowsCrs {
+  const int *ptr, *index;
+  const double *value;
+  __device__ int begin(int i) const { return ptr[i]; }
+  __device__ int end(int i) const { return ptr[i + 1]; }
+  __device__ int col(int, int j) const { return index[j]; }
+  __device__ double val(int, int j) const { return value[j]; }
+};
+struct RowsEll {
+  const int *length, *index;
+  const double *data;
+  int width;
+  __device__ int begin(int) const { return 0; }
+  __device__ int end(int i) const { return length[i]; }
+  __device__ int col(int i, int j) const { return index[ell_at(i, j, width)]; }
+  __device__ double val(int i, int j) const { return data[ell_at(i, j, width)]; }
+};
+
 // Distinct offsets col - row of all entries, collected per CTA in shared
 // memory and merged into the global table. *flag |= 1 on overflow.
+template <typename Rows>
 __global__ void __launch_bounds__(kThreads)
-    k_band_offsets(int N, const int *__restrict__ ptr, const int *__restrict__ col,
-                   int *table, int *flag) {
+    k_band_offsets(int N, Rows A, int *table, int *flag) {
   __shared__ int local[kBandTable];
   __shared__ int full;
   if (threadIdx.x < kBandTable) local[threadIdx.x] = kBandEmpty;
   if (threadIdx.x == 0) full = 0;
   __syncthreads();
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < N; i += gridDim.x * kThreads) {
-    const int j1 = ptr[i + 1];
-    for (int j = ptr[i]; j < j1; j++)
-      if (!band_insert(local, col[j] - i)) {
+    const int j1 = A.end(i);
+    for (int j = A.begin(i); j < j1; j++)
+      if (!band_insert(local, A.col(i, j) - i)) {
         full = 1;
         break;
       }

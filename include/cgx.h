@@ -77,23 +77,28 @@ typedef enum cgx_precision {
 } cgx_precision;
 
 typedef enum cgx_loop {
-  CGX_LOOP_GRAPH = 0,   /* whole solve = one CUDA graph with a while node;
-                           the mixed paths on the band form run their inner
-                           solves as persistent launches below (PERSISTENT up
-                           to 1.3M rows, PERSISTENT_SPLIT beyond), which
-                           measured faster at every size */
+  CGX_LOOP_GRAPH = 0,   /* whole solve = one CUDA graph with a while node,
+                           or, on structured-grid matrices, the persistent
+                           launches below where they measured faster: the
+                           mixed paths' inner solves on the band form, and
+                           plain FP64 solves of matrices with sorted rows and
+                           at most 27 column offsets */
   CGX_LOOP_CHUNKED = 1, /* graph of a fixed number of iterations, host polls */
   CGX_LOOP_KERNELS = 2, /* one launch per fused kernel, each timed by events */
   CGX_LOOP_PERSISTENT = 3, /* mixed paths on the band form (the 7- and
                            5-point stencils, any size): each inner solve is
                            one cooperative launch whose fused phases (three
                            per learned iteration, two per Jacobi one) meet at
-                           grid-wide barriers; other solves run as GRAPH */
+                           grid-wide barriers; a plain FP64 solve of a matrix
+                           with sorted rows and at most 27 column offsets is
+                           one such launch too (two phases); other solves run
+                           as GRAPH */
   CGX_LOOP_PERSISTENT_SPLIT = 4 /* the same launch with one phase per kernel
                            of the GRAPH iteration (five learned, three
-                           Jacobi) and no value formed twice; also on SELL-U
-                           inner products whose slices are all uniform (the
-                           27-point stencils), where GRAPH takes it too */
+                           Jacobi or plain FP64) and no value formed twice;
+                           also on SELL-U inner products whose slices are all
+                           uniform (the 27-point stencils), where GRAPH takes
+                           it too */
 } cgx_loop;
 
 /* Solver settings: the reference's CG_* environment switches

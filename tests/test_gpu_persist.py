@@ -103,3 +103,112 @@ def test_sell_form_agrees_with_the_kernels(handle, N, learned):
     x = out[cg.LOOP_KERNELS][1]
     # 12 on the diagonal, five offsets: eigenvalues in [2, 22].
     assert np.linalg.norm(out[cg.LOOP_GRAPH][1] - x) <= 2 * tol * 11 * np.linalg.norm(x)
+
+
+def fp64_matrix(kind, N):
+    """Matrices of each form the plain persistent solve stores, and two that
+    it must leave to the rows."""
+    if kind == "half3":  # up to 3 non-negative offsets
+        return band_matrix(N, (1, 61))
+    if kind == "half4":
+        return band_matrix(N, (1, 61, 1777))
+    if kind == "half14":
+        A = band_matrix(N, (1, 2, 31, 32, 33, 901, 931, 932, 933, 962, 963, 964, 965))
+        A.value[A.rows() == A.index] += 20.0
+        return A
+    A = band_matrix(N, (1, 61, 1777) if kind in ("all7", "reversed")
+                    else (1, 2, 31, 32, 33, 901, 931, 932, 933, 962, 963, 964, 965))
+    if kind == "all27":
+        A.value[A.rows() == A.index] += 20.0
+    if kind in ("all7", "all27") and A.nz > A.N:
+        # Not symmetric in the last bit of one entry: every offset is stored.
+        k = np.flatnonzero(A.rows() != A.index)[0]
+        A.value[k] = np.nextafter(A.value[k], 0.0)
+    if kind == "reversed":  # columns descend: not the order of the offsets
+        order = np.lexsort((-A.index, A.rows()))
+        A = G.Crs(A.N, A.ptr, A.index[order].copy(), A.value[order].copy())
+    if kind == "sparse":  # 27 offsets, most of them empty
+        keep = (A.rows() == A.index) | ((A.rows() + A.index) % 16 == 0)
+        rows, cols, vals = A.rows()[keep], A.index[keep], A.value[keep]
+        A = G.crs_from_unsorted(N, rows, cols, vals)
+    return A
+
+
+KINDS = ["half3", "half4", "half14", "all7", "all27", "reversed", "sparse"]
+
+
+def upload(handle, A, fmt):
+    if fmt == "ell":
+        handle.upload_ell(A.N, A.nz, *G.to_ell(A))
+    elif fmt == "coo":
+        handle.upload_coo(A.N, A.rows(), A.index, A.value)
+    else:
+        handle.upload_crs(A.ptr, A.index, A.value)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("N", [1, 2, 33, 255, 257, 1025, 4098, 37889, 75777, 151553])
+def test_plain_forms_agree_with_the_kernels(handle, kind, N):
+    """Ten iterations of every form against the chunked kernels. The forms
+    differ in the order of the dot products' sums only: a relative error of at
+    most N * 2^-53 in each, 20 of them, and as the iterates depend smoothly on
+    the scalars (condition at most 7), at most 20 * 7 * N * 2^-53 in x."""
+    A = fp64_matrix(kind, N)
+    b, _ = G.rhs_for(A, seed=3)
+    fmt = ("crs", "ell", "coo")[(N + len(kind)) % 3]
+    upload(handle, A, fmt)
+    handle.jacobi_from_matrix()
+    handle.set_vector("K", b)
+    for pc in (cg.PRECOND_JACOBI, cg.PRECOND_NONE):
+        out = {}
+        for loop in (cg.LOOP_CHUNKED, cg.LOOP_GRAPH, cg.LOOP_PERSISTENT,
+                     cg.LOOP_PERSISTENT_SPLIT):
+            handle.fill_vector("X", 0.25)
+            r = handle.solve(max_iterations=10, tolerance=1e-30, preconditioner=pc, loop=loop)
+            out[loop] = (r, [handle.get_vector(v) for v in "XRPQ"])
+        r0, v0 = out[cg.LOOP_CHUNKED]
+        if not np.isfinite(v0[0]).all() or r0["residual"] < 1e-12:
+            continue  # converged to zero: the last iterates are rounding noise
+        bound = 20 * KAPPA * N * 2.0 ** -53
+        for loop in (cg.LOOP_GRAPH, cg.LOOP_PERSISTENT, cg.LOOP_PERSISTENT_SPLIT):
+            r, v = out[loop]
+            assert r["iterations"] == r0["iterations"] == 10, (loop, r)
+            assert r["converged"] == 0
+            for name, a, c in zip("XRPQ", v, v0):
+                scale = max(np.linalg.norm(c), np.linalg.norm(v0[0]) * 1e-3)
+                assert np.linalg.norm(a - c) <= bound * scale + 1e-300, (loop, pc, name)
+
+
+@pytest.mark.parametrize("loop", [cg.LOOP_GRAPH, cg.LOOP_PERSISTENT, cg.LOOP_PERSISTENT_SPLIT])
+def test_plain_forms_stop_as_the_kernels_do(handle, loop):
+    """Convergence, the iteration limit, a NaN that never converges, and new
+    values on the same pattern."""
+    A = band_matrix(5003, (1, 61, 1777))
+    b, xs = G.rhs_for(A, seed=4)
+    handle.upload_crs(A.ptr, A.index, A.value)
+    handle.jacobi_from_matrix()
+    handle.set_vector("K", b)
+    want = {}
+    for lp in (cg.LOOP_CHUNKED, loop):
+        handle.fill_vector("X", 0.0)
+        r = handle.solve(max_iterations=1000, tolerance=1e-11, loop=lp)
+        want[lp] = r["iterations"]
+        assert r["converged"] == 1 and r["residual"] <= 1e-11
+        assert np.linalg.norm(handle.get_vector("X") - xs) <= 1e-11 * KAPPA * np.linalg.norm(xs)
+    assert want[loop] == want[cg.LOOP_CHUNKED]
+    handle.fill_vector("X", 0.0)
+    r = handle.solve(max_iterations=1, tolerance=1e-11, loop=loop)
+    assert r["iterations"] == 1 and r["converged"] == 0
+    v = 3.0 * A.value
+    handle.update_crs_values(v)
+    handle.jacobi_from_matrix()
+    handle.fill_vector("X", 0.0)
+    r = handle.solve(max_iterations=1000, tolerance=1e-11, loop=loop)
+    assert r["converged"] == 1
+    assert np.linalg.norm(3.0 * handle.get_vector("X") - xs) <= 1e-11 * KAPPA * np.linalg.norm(xs)
+    bad = b.copy()
+    bad[17] = np.nan
+    handle.set_vector("K", bad)
+    handle.fill_vector("X", 0.0)
+    r = handle.solve(max_iterations=7, tolerance=1e-11, loop=loop)
+    assert r["iterations"] == 7 and r["converged"] == 0
