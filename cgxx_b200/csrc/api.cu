@@ -32,6 +32,7 @@
 #include "persist.cuh"
 #include "sell.cuh"
 #include "solve64.cuh"
+#include "train.cuh"
 
 using namespace cgx;
 
@@ -286,16 +287,14 @@ struct Learned {
   bool gb_ok = false;
   __nv_bfloat16 *h[4] = {};
   __nv_bfloat16 *agg[3] = {};
-  float *pre[4] = {};
+  uint32_t *pos[4] = {};  // bit masks of positive pre-activations
   float *o = nullptr;
   float *y32 = nullptr, *z32 = nullptr;
   // training
   float *V = nullptr, *T1 = nullptr, *T2 = nullptr, *rho = nullptr;
-  float *dT2 = nullptr, *dT1 = nullptr, *dg = nullptr, *dO = nullptr;
-  float *dh = nullptr, *dh2 = nullptr, *dself = nullptr, *dagg = nullptr,
-        *dpre = nullptr;
+  float *dT2 = nullptr, *dT1 = nullptr, *cfac = nullptr, *dO = nullptr;
+  float *dself[2] = {}, *dagg[2] = {};  // in turn, layer after layer
   float *partial = nullptr, *grad = nullptr, *loss = nullptr;
-  float *gtmp = nullptr;  // two reduced [W*W | W] blocks of a layer gradient
   float *snap = nullptr;  // residual snapshots (probe columns), N x S
   double *snap_scale = nullptr;
   unsigned snap_valid = 0;  // bit c: column c holds a snapshot of this matrix
@@ -2737,6 +2736,9 @@ cgx_status learned_alloc(cgx_handle *h, int nnzL) {
   return CGX_SUCCESS;
 }
 
+// CTAs of the backward kernels: one wave, and a row of partial sums each.
+int back_grid(const cgx_handle *h) { return h->num_sms * kBackCtas; }
+
 cgx_status learned_train_alloc(cgx_handle *h) {
   Learned *L = h->L;
   if (L->train) return CGX_SUCCESS;
@@ -2745,17 +2747,16 @@ cgx_status learned_train_alloc(cgx_handle *h) {
   size_t o[20];
   int k = 0;
   for (int q = 0; q < 7; q++) o[k++] = take_n<float>(c, (size_t)N * S);
-  o[k++] = take_n<float>(c, L->nnzL);                 // dg
+  o[k++] = take_n<float>(c, L->nnzL);                 // cfac
   o[k++] = take_n<float>(c, (size_t)N * NOUT);        // dO
-  for (int q = 0; q < 5; q++) o[k++] = take_n<float>(c, (size_t)N * W);
-  o[k++] = take_n<float>(c, (size_t)kMaxGrid * (W * 2 * W + W));  // partial
+  for (int q = 0; q < 4; q++) o[k++] = take_n<float>(c, (size_t)N * W);
+  o[k++] = take_n<float>(c, (size_t)back_grid(h) * NPARAMS);  // partial
   o[k++] = take_n<float>(c, NPARAMS);                 // grad
   o[k++] = take_n<float>(c, 4);                       // loss
-  o[k++] = take_n<float>(c, 2 * (W * W + W));         // gtmp
   o[k++] = take_n<double>(c, 1);                      // snap_scale
-  size_t o_agg[3], o_pre[4];
+  size_t o_agg[3], o_pos[4];
   for (int q = 0; q < 3; q++) o_agg[q] = take_n<__nv_bfloat16>(c, (size_t)N * W);
-  for (int q = 0; q < 4; q++) o_pre[q] = take_n<float>(c, (size_t)N * W);
+  for (int q = 0; q < 4; q++) o_pos[q] = take_n<uint32_t>(c, (size_t)N);
   CUDA_TRY(dev_alloc(h, (void **)&L->train, c.off));
   CUDA_TRY(cudaMemsetAsync(L->train, 0, c.off, h->stream));
   char *b = (char *)L->train;
@@ -2767,20 +2768,16 @@ cgx_status learned_train_alloc(cgx_handle *h) {
   L->dT2 = (float *)(b + o[k++]);
   L->dT1 = (float *)(b + o[k++]);
   L->snap = (float *)(b + o[k++]);
-  L->dg = (float *)(b + o[k++]);
+  L->cfac = (float *)(b + o[k++]);
   L->dO = (float *)(b + o[k++]);
-  L->dh = (float *)(b + o[k++]);
-  L->dh2 = (float *)(b + o[k++]);
-  L->dself = (float *)(b + o[k++]);
-  L->dagg = (float *)(b + o[k++]);
-  L->dpre = (float *)(b + o[k++]);
+  for (int q = 0; q < 2; q++) L->dself[q] = (float *)(b + o[k++]);
+  for (int q = 0; q < 2; q++) L->dagg[q] = (float *)(b + o[k++]);
   L->partial = (float *)(b + o[k++]);
   L->grad = (float *)(b + o[k++]);
   L->loss = (float *)(b + o[k++]);
-  L->gtmp = (float *)(b + o[k++]);
   L->snap_scale = (double *)(b + o[k++]);
   for (int q = 0; q < 3; q++) L->agg[q] = (__nv_bfloat16 *)(b + o_agg[q]);
-  for (int q = 0; q < 4; q++) L->pre[q] = (float *)(b + o_pre[q]);
+  for (int q = 0; q < 4; q++) L->pos[q] = (uint32_t *)(b + o_pos[q]);
   return CGX_SUCCESS;
 }
 
@@ -2914,11 +2911,11 @@ cudaError_t gnn_forward(cgx_handle *h, const float *P, bool scaled) {
   Learned *L = h->L;
   const int N = h->N;
   cudaStream_t s = h->stream;
-  // Inference (scaled) keeps no pre-activations or aggregates: only the
-  // backward pass needs them.
+  // Inference (scaled) keeps no masks or aggregates: only the backward pass
+  // needs them.
   const bool keep = !scaled;
   k_embed<<<grid_for(h, (size_t)N), kThreads, 0, s>>>(
-      N, L->feat, P, L->h[0], keep ? L->pre[0] : nullptr);
+      N, L->feat, P, L->h[0], keep ? L->pos[0] : nullptr);
   const int groups = (N + 15) / 16;
   const int lgrid = std::max(
       1, std::min(h->num_sms * 8, (groups + kLayerWarps - 1) / kLayerWarps));
@@ -2926,7 +2923,7 @@ cudaError_t gnn_forward(cgx_handle *h, const float *P, bool scaled) {
     k_layer<<<lgrid, 32 * kLayerWarps, 0, s>>>(N, h->ptr, h->index, L->ahat, P,
                                                l, L->h[l], L->h[l + 1],
                                                keep ? L->agg[l] : nullptr,
-                                               keep ? L->pre[l + 1] : nullptr);
+                                               keep ? L->pos[l + 1] : nullptr);
   k_head<<<grid_for(h, (size_t)N), kThreads, 0, s>>>(N, L->h[3], P, L->o);
   k_assemble<<<grid_for(h, L->nnzL), kThreads, 0, s>>>(
       L->nnzL, L->grow, L->gcol, L->g2a, L->ahat, L->o, L->ghat, L->dis,
@@ -2942,53 +2939,31 @@ cudaError_t gnn_backward(cgx_handle *h, const float *P) {
   Learned *L = h->L;
   const int N = h->N;
   cudaStream_t s = h->stream;
-  const int g = grid_for(h, N);
+  const int g = grid_for(h, 2 * (size_t)N);  // two lanes per node
   // T1 = Ghat V, T2 = Ahat T1, R = Ghat^T T2 - V.
-  k_spmm8<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->ghat, nullptr, L->V, L->T1);
-  k_spmm8<<<g, kThreads, 0, s>>>(N, h->ptr, h->index, L->ahat, nullptr, L->T1, L->T2);
+  k_spmm8<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->ghat, L->V, L->T1);
+  k_spmm8<<<g, kThreads, 0, s>>>(N, h->ptr, h->index, L->ahat, L->T1, L->T2);
   k_loss_residual<<<g, kThreads, 0, s>>>(N, L->tptr, L->tcol, L->ghat, L->t2g,
                                          L->T2, L->V, L->rho, h->partials,
                                          ticket(h, kTicketDot), L->loss);
-  // dT2 = Ghat rho, dT1 = Ahat dT2, dGhat.
-  k_spmm8<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->ghat, nullptr, L->rho, L->dT2);
-  k_spmm8<<<g, kThreads, 0, s>>>(N, h->ptr, h->index, L->ahat, nullptr, L->dT2, L->dT1);
-  k_grad_factor<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->T2, L->dT1, L->rho,
-                                       L->V, L->dg);
-  k_grad_head_out<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->g2a, L->tptr,
-                                         L->tcol, L->t2g, L->ahat, L->o, L->dg,
-                                         L->dO);
-  const int pg = std::max(1, std::min(kMaxGrid, (N + 31) / 32));
-  // Head weights: dW_h = sum dO h3^T, db_h = sum dO.
-  k_outer_partials<NOUT, W, __nv_bfloat16><<<pg, kThreads, 0, s>>>(
-      N, L->dO, L->h[3], L->partial);
-  k_reduce_partials<<<grid_for(h, NOUT * W + NOUT), kThreads, 0, s>>>(
-      pg, NOUT * W + NOUT, L->partial, L->grad + OFF_WH);
-  k_grad_head_in<<<grid_for(h, (size_t)N * W), kThreads, 0, s>>>(N, P, L->dO, L->dh);
-  // Layers 2..0.
-  float *dcur = L->dh, *dnext = L->dh2;
-  for (int l = 2; l >= 0; l--) {
-    k_layer_back1<<<grid_for(h, (size_t)N * W), kThreads, 0, s>>>(
-        N, P, l, dcur, L->pre[l + 1], L->dpre, L->dself, L->dagg);
-    // dW_l[:, 0:W] = sum dpre h_l^T (+ bias), dW_l[:, W:2W] = sum dpre agg^T.
-    k_outer_partials<W, W, __nv_bfloat16><<<pg, kThreads, 0, s>>>(
-        N, L->dpre, L->h[l], L->partial);
-    k_reduce_partials<<<grid_for(h, W * W + W), kThreads, 0, s>>>(
-        pg, W * W + W, L->partial, L->gtmp);
-    k_outer_partials<W, W, __nv_bfloat16><<<pg, kThreads, 0, s>>>(
-        N, L->dpre, L->agg[l], L->partial);
-    k_reduce_partials<<<grid_for(h, W * W + W), kThreads, 0, s>>>(
-        pg, W * W + W, L->partial, L->gtmp + (W * W + W));
-    k_pack_layer_grad<<<1, kThreads, 0, s>>>(L->gtmp, L->grad + OFF_L0 + l * L_STRIDE);
-    k_layer_back2<<<grid_for(h, (size_t)N * 32), kThreads, 0, s>>>(
-        N, h->ptr, h->index, L->ahat, L->dself, L->dagg, dnext);
-    std::swap(dcur, dnext);
-  }
-  // Embedding.
-  k_relu_back<<<grid_for(h, (size_t)N * W), kThreads, 0, s>>>(N * W, L->pre[0], dcur);
-  k_outer_partials<W, NIN, float><<<pg, kThreads, 0, s>>>(N, dcur, L->feat,
-                                                          L->partial);
-  k_reduce_partials<<<grid_for(h, W * NIN + W), kThreads, 0, s>>>(
-      pg, W * NIN + W, L->partial, L->grad + OFF_WIN);
+  // dT2 = Ghat rho, dT1 = Ahat dT2, dGhat and the head outputs.
+  k_spmm8<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->ghat, L->rho, L->dT2);
+  k_spmm8<<<g, kThreads, 0, s>>>(N, h->ptr, h->index, L->ahat, L->dT2, L->dT1);
+  k_grad_rows<<<g, kThreads, 0, s>>>(N, L->gptr, L->gcol, L->g2a, L->ahat, L->T2, L->dT1,
+                                     L->rho, L->V, L->o, L->cfac, L->dO);
+  k_grad_cols<<<g, kThreads, 0, s>>>(N, L->tptr, L->tcol, L->t2g, L->cfac, L->o, L->dO);
+  // The layers from the last (with the head), the embedding, the sums.
+  const int bg = back_grid(h);
+  k_layer_back<true><<<bg, 32 * kBackWarps, 0, s>>>(
+      N, h->ptr, h->index, L->ahat, P, 2, L->dO, L->h[3], nullptr, nullptr, L->pos[3], L->h[2],
+      L->agg[2], L->dself[0], L->dagg[0], L->partial);
+  for (int l = 1; l >= 0; l--)
+    k_layer_back<false><<<bg, 32 * kBackWarps, 0, s>>>(
+        N, h->ptr, h->index, L->ahat, P, l, nullptr, nullptr, L->dself[1 - l], L->dagg[1 - l],
+        L->pos[l + 1], L->h[l], L->agg[l], L->dself[l], L->dagg[l], L->partial);
+  k_embed_back<<<bg, kEmbedBackThreads, 0, s>>>(N, h->ptr, h->index, L->ahat, L->dself[0],
+                                                L->dagg[0], L->pos[0], L->feat, L->partial);
+  k_sum_partials<<<(NPARAMS + 31) / 32, kThreads, 0, s>>>(bg, L->partial, L->grad);
   return cudaGetLastError();
 }
 
@@ -3325,11 +3300,10 @@ static cgx_status make_probes(const cgx_gnn *gn, cgx_handle *h,
   const int gs = grid_stream(h, (size_t)h->N * S);
   k_rademacher<<<gs, kThreads, 0, s>>>(h->N, seed, L->V);
   for (int k = 0; k < gn->smooth_steps && c1 > c0; k++) {
-    k_spmm8<<<grid_stream(h, h->N), kThreads, 0, s>>>(h->N, h->ptr, h->index,
-                                                       L->ahat, nullptr, L->V, L->T1);
-    k_smooth_probes<<<gs, kThreads, 0, s>>>(
-        h->N, L->V, L->T1, 2.f / 3.f,
-        k == gn->smooth_steps - 1 ? gn->smooth_scale : 1.f, c0, c1);
+    k_smooth8<<<grid_stream(h, 2 * (size_t)h->N), kThreads, 0, s>>>(
+        h->N, h->ptr, h->index, L->ahat, 2.f / 3.f,
+        k == gn->smooth_steps - 1 ? gn->smooth_scale : 1.f, c0, c1, L->V, L->T1);
+    std::swap(L->V, L->T1);
   }
   if (rc > 0) k_copy_probe_cols<<<gs, kThreads, 0, s>>>(h->N, L->snap, L->V, c1);
   CUDA_TRY(cudaGetLastError());

@@ -5,11 +5,7 @@
 //     order) and of G^T (upper triangle), and the maps between them;
 //   - the message-passing network that emits G's values (forward on BF16
 //     tensor cores, mma.sync m16n8k16, FP32 accumulation);
-//   - its training: the Hutchinson loss ||(Ghat^T Ahat Ghat - I) V||^2 and the
-//     backward pass through the factor, the head, the three layers and the
-//     embedding (gathers over the symmetric pattern; no atomics, so the
-//     gradient is deterministic);
-//   - Adam.
+//   - Adam and the training probes (the loss and the backward pass: train.cuh).
 // The exact arithmetic is stated in oracle/gnn_oracle.py, the CPU oracle the
 // tests compare these kernels with.
 #pragma once
@@ -207,10 +203,12 @@ __global__ void k_transpose_map(int nnzL, const int *__restrict__ grow,
 
 __device__ __forceinline__ float relu(float x) { return x > 0.f ? x : 0.f; }
 
-// h0 = bf16(relu(W_in f + b_in)); also keeps pre0 for the backward pass.
+// h0 = bf16(relu(W_in f + b_in)). For the backward pass: bit f of mask[i] says
+// that pre-activation f of node i is positive, which is all that it reads of
+// them (4 bytes per node and layer instead of 128).
 __global__ void k_embed(int N, const float *__restrict__ feat,
                         const float *__restrict__ P, __nv_bfloat16 *__restrict__ h,
-                        float *__restrict__ pre) {
+                        uint32_t *__restrict__ mask) {
   // One thread per node: W_in and b_in (contiguous in P) from shared memory,
   // the node's 4 features in one 16-byte load, its 32 outputs in four
   // 16-byte stores.
@@ -223,14 +221,16 @@ __global__ void k_embed(int N, const float *__restrict__ feat,
     const float fv[NIN] = {f4.x, f4.y, f4.z, f4.w};
     uint4 out[W / 8];
     __nv_bfloat16 *ob = reinterpret_cast<__nv_bfloat16 *>(out);
+    uint32_t bits = 0u;
 #pragma unroll
     for (int f = 0; f < W; f++) {
       float s = sW[W * NIN + f];
 #pragma unroll
       for (int k = 0; k < NIN; k++) s = fmaf(sW[f * NIN + k], fv[k], s);
-      if (pre) pre[(size_t)i * W + f] = s;
+      bits |= s > 0.f ? 1u << f : 0u;
       ob[f] = __float2bfloat16_rn(relu(s));
     }
+    if (mask) mask[i] = bits;
     uint4 *dst = reinterpret_cast<uint4 *>(h + (size_t)i * W);
 #pragma unroll
     for (int q = 0; q < W / 8; q++) dst[q] = out[q];
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(32 * kLayerWarps)
             const float *__restrict__ ahat, const float *__restrict__ P,
             int layer, const __nv_bfloat16 *__restrict__ hin,
             __nv_bfloat16 *__restrict__ hout, __nv_bfloat16 *__restrict__ agg_out,
-            float *__restrict__ pre_out) {
+            uint32_t *__restrict__ mask_out) {
   __shared__ __align__(16) __nv_bfloat16 sW[W][2 * W + 8];  // W_l[n][k], rows padded (banks)
   __shared__ __align__(16) __nv_bfloat16 sX[kLayerWarps][16][2 * W + 8];  // padded rows
   __shared__ float sB[W];
@@ -301,22 +301,19 @@ __global__ void __launch_bounds__(32 * kLayerWarps)
           uint4 hv[4];
           int cc[4];
           // All four entries' columns and weights first, then the four
-          // gathers: one round trip for each instead of one per entry
-          // (measured: inference 6 % faster at 160^3).
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-            if (j + u < j1) {
-              cc[u] = index[j + u];
-              w[u] = fabsf(ahat[j + u]);
-            }
+          // gathers: one round trip for each instead of one per entry. The
+          // loads are unconditional (past the row's end: its last entry again,
+          // weight 0), as a condition would make each a branch.
 #pragma unroll
           for (int u = 0; u < 4; u++) {
-            if (j + u < j1) {
-              const int c = cc[u];
-              w[u] = c != i ? w[u] : 0.f;
-              hv[u] = hin4[(size_t)c * (W / 8) + c4];
-            }
+            const int e = min(j + u, j1 - 1);
+            cc[u] = index[e];
+            w[u] = fabsf(ahat[e]);
           }
+#pragma unroll
+          for (int u = 0; u < 4; u++) hv[u] = hin4[(size_t)cc[u] * (W / 8) + c4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) w[u] = cc[u] != i ? w[u] : 0.f;
 #pragma unroll
           for (int u = 0; u < 4; u++) {
             if (j + u < j1) {
@@ -368,6 +365,7 @@ __global__ void __launch_bounds__(32 * kLayerWarps)
     // replaces h_i in the staging rows (each element is read and written by
     // the lane that owns it), then the warp stores its 16 rows as 16-byte
     // chunks.
+    uint32_t pos[2] = {0u, 0u};  // positive pre-activations of rows g, g + 8
 #pragma unroll
     for (int nt = 0; nt < 4; nt++)
 #pragma unroll
@@ -375,10 +373,18 @@ __global__ void __launch_bounds__(32 * kLayerWarps)
         const int r = g + (q >= 2 ? 8 : 0);
         const int col = nt * 8 + 2 * tq + (q & 1);
         const float pre = acc[nt][q] + sB[col];
-        if (pre_out && base + r < N) pre_out[(size_t)(base + r) * W + col] = pre;
+        pos[q >> 1] |= pre > 0.f ? 1u << col : 0u;
         const float hv = __bfloat162float(sX[warp][r][col]) + relu(pre);
         sX[warp][r][col] = __float2bfloat16_rn(hv);
       }
+    if (mask_out) {
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        pos[k] |= __shfl_xor_sync(0xffffffffu, pos[k], 1);
+        pos[k] |= __shfl_xor_sync(0xffffffffu, pos[k], 2);
+        if (tq == 0 && base + g + 8 * k < N) mask_out[base + g + 8 * k] = pos[k];
+      }
+    }
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -472,316 +478,7 @@ __global__ void k_assemble(int nnzL, const int *__restrict__ grow,
 }
 
 // ---------------------------------------------------------------------------
-// Training: Hutchinson loss with S probe columns (node-major: V[i*S + s])
-
-__device__ __forceinline__ void load8(const float *p, float (&v)[S]) {
-  const float4 a = *reinterpret_cast<const float4 *>(p);
-  const float4 b = *reinterpret_cast<const float4 *>(p + 4);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void store8(float *p, const float (&v)[S]) {
-  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-  *reinterpret_cast<float4 *>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
-}
-
-// OUT = M IN for an S-column block, M in CRS with values val[map[e]] (map may
-// be null: val[e]).
-__global__ void k_spmm8(int N, const int *__restrict__ rp,
-                        const int *__restrict__ col, const float *__restrict__ val,
-                        const int *__restrict__ map, const float *__restrict__ in,
-                        float *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += gridDim.x * blockDim.x) {
-    float acc[S] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int e = rp[i]; e < rp[i + 1]; e++) {
-      const float a = val[map ? map[e] : e];
-      float v[S];
-      load8(in + (size_t)col[e] * S, v);
-#pragma unroll
-      for (int s = 0; s < S; s++) acc[s] = fmaf(a, v[s], acc[s]);
-    }
-    store8(out + (size_t)i * S, acc);
-  }
-}
-
-// T3 = G^T T2 (G^T rows with values ghat[t2g[t]]), R = T3 - V,
-// rho = 2 R / (N S), partial sums of R^2 -> *loss (last CTA).
-__global__ void __launch_bounds__(kThreads)
-    k_loss_residual(int N, const int *__restrict__ tptr,
-                    const int *__restrict__ tcol, const float *__restrict__ ghat,
-                    const int *__restrict__ t2g, const float *__restrict__ T2,
-                    const float *__restrict__ V, float *__restrict__ rho,
-                    double *partials, unsigned *ticket, float *loss) {
-  const float scale = 2.f / ((float)N * S);
-  double acc = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += gridDim.x * blockDim.x) {
-    float t3[S] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int e = tptr[i]; e < tptr[i + 1]; e++) {
-      const float a = ghat[t2g[e]];
-      float v[S];
-      load8(T2 + (size_t)tcol[e] * S, v);
-#pragma unroll
-      for (int s = 0; s < S; s++) t3[s] = fmaf(a, v[s], t3[s]);
-    }
-    float v[S], r[S];
-    load8(V + (size_t)i * S, v);
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-      const float d = t3[s] - v[s];
-      acc += (double)d * d;
-      r[s] = scale * d;
-    }
-    store8(rho + (size_t)i * S, r);
-  }
-  double in[1] = {acc}, out[1];
-  if (grid_reduce<1>(in, partials, ticket, out) && threadIdx.x == 0)
-    *loss = (float)(out[0] / ((double)N * S));
-}
-
-// dGhat for every G entry e = (i, j): sum_s T2[i,s] rho[j,s] + dT1[i,s] V[j,s].
-__global__ void k_grad_factor(int N, const int *__restrict__ gptr,
-                              const int *__restrict__ gcol,
-                              const float *__restrict__ T2,
-                              const float *__restrict__ dT1,
-                              const float *__restrict__ rho,
-                              const float *__restrict__ V,
-                              float *__restrict__ dg) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += gridDim.x * blockDim.x) {
-    float t2[S], d1[S];
-    load8(T2 + (size_t)i * S, t2);
-    load8(dT1 + (size_t)i * S, d1);
-    for (int e = gptr[i]; e < gptr[i + 1]; e++) {
-      const int j = gcol[e];
-      float r[S], v[S];
-      load8(rho + (size_t)j * S, r);
-      load8(V + (size_t)j * S, v);
-      float s = 0.f;
-#pragma unroll
-      for (int q = 0; q < S; q++) s = fmaf(t2[q], r[q], fmaf(d1[q], v[q], s));
-      dg[e] = s;
-    }
-  }
-}
-
-// Gradient w.r.t. the head outputs o_i = [a, dg, u, v]:
-//   d dg_i = dGhat_ii sigmoid(dg_i + offset)
-//   d a_i  = sum_{(i,j), j<i} dGhat_ij w_ij
-//   d u_i  = sum_{(i,j), j<i} dGhat_ij w_ij v_j
-//   d v_j  = sum_{(i,j), i>j} dGhat_ij w_ij u_i   (over row j of G^T)
-__global__ void k_grad_head_out(int N, const int *__restrict__ gptr,
-                                const int *__restrict__ gcol,
-                                const int *__restrict__ g2a,
-                                const int *__restrict__ tptr,
-                                const int *__restrict__ tcol,
-                                const int *__restrict__ t2g,
-                                const float *__restrict__ ahat,
-                                const float *__restrict__ o,
-                                const float *__restrict__ dg,
-                                float *__restrict__ dO) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += gridDim.x * blockDim.x) {
-    float da = 0.f, ddg = 0.f, du[RANK] = {0.f, 0.f, 0.f, 0.f},
-          dv[RANK] = {0.f, 0.f, 0.f, 0.f};
-    for (int e = gptr[i]; e < gptr[i + 1]; e++) {
-      const int j = gcol[e];
-      if (j == i) {
-        ddg += dg[e] * sigmoid(o[i * NOUT + 1] + DIAG_OFFSET);
-      } else {
-        const float c = dg[e] * fabsf(ahat[g2a[e]]);
-        da += c;
-#pragma unroll
-        for (int k = 0; k < RANK; k++)
-          du[k] = fmaf(c, o[j * NOUT + 2 + RANK + k], du[k]);
-      }
-    }
-    for (int t = tptr[i]; t < tptr[i + 1]; t++) {
-      const int r = tcol[t];  // G entry (r, i), r > i
-      if (r == i) continue;
-      const int e = t2g[t];
-      const float c = dg[e] * fabsf(ahat[g2a[e]]);
-#pragma unroll
-      for (int k = 0; k < RANK; k++) dv[k] = fmaf(c, o[r * NOUT + 2 + k], dv[k]);
-    }
-    float *d = dO + (size_t)i * NOUT;
-    d[0] = da;
-    d[1] = ddg;
-#pragma unroll
-    for (int k = 0; k < RANK; k++) {
-      d[2 + k] = du[k];
-      d[2 + RANK + k] = dv[k];
-    }
-  }
-}
-
-// dh_i = W_h^T dO_i (FP32).
-__global__ void k_grad_head_in(int N, const float *__restrict__ P,
-                               const float *__restrict__ dO,
-                               float *__restrict__ dh) {
-  const int total = N * W;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += gridDim.x * blockDim.x) {
-    const int i = t / W, f = t % W;
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < NOUT; k++)
-      s = fmaf(P[OFF_WH + k * W + f], dO[(size_t)i * NOUT + k], s);
-    dh[t] = s;
-  }
-}
-
-__device__ __forceinline__ float to_f(float v) { return v; }
-__device__ __forceinline__ float to_f(__nv_bfloat16 v) {
-  return __bfloat162float(v);
-}
-
-// Per-CTA partial sums of a_i b_i^T (NA x NB) and of a_i (NA), for weight
-// and bias gradients: partial[blockIdx.x][NA*NB + NA]. Rows of a and b are
-// contiguous (lda = NA, ldb = NB). A fixed split of nodes over CTAs and a
-// fixed order inside each makes the sums deterministic.
-template <int NA, int NB, typename TB>
-__global__ void __launch_bounds__(kThreads)
-    k_outer_partials(int N, const float *__restrict__ a,
-                     const TB *__restrict__ b, float *__restrict__ partial) {
-  constexpr int CH = 32;  // nodes per chunk
-  __shared__ float sa[CH][NA];
-  __shared__ float sb[CH][NB];
-  constexpr int NOUTS = NA * NB + NA;
-  constexpr int PER = (NOUTS + kThreads - 1) / kThreads;
-  float acc[PER];
-#pragma unroll
-  for (int q = 0; q < PER; q++) acc[q] = 0.f;
-  const int chunks = (N + CH - 1) / CH;
-  const int per_cta = (chunks + gridDim.x - 1) / gridDim.x;
-  const int c0 = blockIdx.x * per_cta, c1 = min(chunks, c0 + per_cta);
-  for (int c = c0; c < c1; c++) {
-    const int n0 = c * CH;
-    for (int t = threadIdx.x; t < CH * NA; t += kThreads) {
-      const int r = t / NA, k = t % NA, i = n0 + r;
-      sa[r][k] = i < N ? a[(size_t)i * NA + k] : 0.f;
-    }
-    for (int t = threadIdx.x; t < CH * NB; t += kThreads) {
-      const int r = t / NB, k = t % NB, i = n0 + r;
-      sb[r][k] = i < N ? to_f(b[(size_t)i * NB + k]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-      const int o = threadIdx.x + q * kThreads;
-      if (o < NA * NB) {
-        const int fa = o / NB, fb = o % NB;
-        float s = acc[q];
-        for (int r = 0; r < CH; r++) s = fmaf(sa[r][fa], sb[r][fb], s);
-        acc[q] = s;
-      } else if (o < NOUTS) {
-        const int fa = o - NA * NB;
-        float s = acc[q];
-        for (int r = 0; r < CH; r++) s += sa[r][fa];
-        acc[q] = s;
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int q = 0; q < PER; q++) {
-    const int o = threadIdx.x + q * kThreads;
-    if (o < NOUTS) partial[(size_t)blockIdx.x * NOUTS + o] = acc[q];
-  }
-}
-
-// out[k] = sum over CTAs of partial[cta][k], CTA order fixed.
-__global__ void k_reduce_partials(int nparts, int len,
-                                  const float *__restrict__ partial,
-                                  float *__restrict__ out) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < len;
-       k += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int c = 0; c < nparts; c++) s += partial[(size_t)c * len + k];
-    out[k] = s;
-  }
-}
-
-// Layer gradient in parameter layout: W_l[n][k] (k < W from the h block,
-// k >= W from the agg block of tmp, each [W*W | W]) followed by b_l[n].
-__global__ void k_pack_layer_grad(const float *__restrict__ tmp,
-                                  float *__restrict__ out) {
-  for (int t = threadIdx.x; t < W * 2 * W + W; t += blockDim.x) {
-    if (t < W * 2 * W) {
-      const int n = t / (2 * W), k = t % (2 * W);
-      out[t] = k < W ? tmp[n * W + k] : tmp[(W * W + W) + n * W + (k - W)];
-    } else {
-      out[t] = tmp[W * W + (t - W * 2 * W)];
-    }
-  }
-}
-
-// Backward through one layer, part 1 (per node): dpre = dh_out * [pre > 0];
-// dX = bf16(W_l)^T dpre; dself = dh_out + dX[0:W]; dagg = dX[W:2W].
-__global__ void k_layer_back1(int N, const float *__restrict__ P, int layer,
-                              const float *__restrict__ dh_out,
-                              const float *__restrict__ pre,
-                              float *__restrict__ dpre,
-                              float *__restrict__ dself,
-                              float *__restrict__ dagg) {
-  __shared__ float sW[W][2 * W];
-  const float *Wl = P + OFF_L0 + layer * L_STRIDE;
-  for (int t = threadIdx.x; t < W * 2 * W; t += blockDim.x)
-    sW[t / (2 * W)][t % (2 * W)] =
-        __bfloat162float(__float2bfloat16_rn(Wl[t]));
-  __syncthreads();
-  const int total = N * W;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += gridDim.x * blockDim.x)
-    dpre[t] = pre[t] > 0.f ? dh_out[t] : 0.f;
-  // dX_i needs all 32 values of dpre_i, which other threads write: each
-  // thread recomputes them from dh_out and pre instead of synchronising.
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += gridDim.x * blockDim.x) {
-    const int i = t / W, f = t % W;
-    const float *dho = dh_out + (size_t)i * W;
-    const float *pr = pre + (size_t)i * W;
-    float xs = 0.f, xa = 0.f;
-#pragma unroll 8
-    for (int n = 0; n < W; n++) {
-      const float dp = pr[n] > 0.f ? dho[n] : 0.f;
-      xs = fmaf(sW[n][f], dp, xs);
-      xa = fmaf(sW[n][W + f], dp, xa);
-    }
-    dself[t] = dh_out[t] + xs;
-    dagg[t] = xa;
-  }
-}
-
-// Backward through one layer, part 2 (gather): dh_in_j = dself_j +
-// sum_{i != j} |Ahat_ji| dagg_i (the aggregation weights are symmetric).
-__global__ void k_layer_back2(int N, const int *__restrict__ ptr,
-                              const int *__restrict__ index,
-                              const float *__restrict__ ahat,
-                              const float *__restrict__ dself,
-                              const float *__restrict__ dagg,
-                              float *__restrict__ dh_in) {
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int j = warp; j < N; j += nwarps) {
-    float s = dself[(size_t)j * W + lane];
-    for (int e = ptr[j]; e < ptr[j + 1]; e++) {
-      const int i = index[e];
-      if (i != j) s = fmaf(fabsf(ahat[e]), dagg[(size_t)i * W + lane], s);
-    }
-    dh_in[(size_t)j * W + lane] = s;
-  }
-}
-
-// Embedding backward: dpre0 = dh0 * [pre0 > 0] (in place).
-__global__ void k_relu_back(int total, const float *__restrict__ pre,
-                            float *__restrict__ d) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += gridDim.x * blockDim.x)
-    if (!(pre[t] > 0.f)) d[t] = 0.f;
-}
+// Training: Adam, probes (the loss and its gradient: train.cuh)
 
 // Adam (bias-corrected), in place.
 __global__ void k_adam(int n, float *__restrict__ p, float *__restrict__ m,
@@ -797,20 +494,6 @@ __global__ void k_adam(int n, float *__restrict__ p, float *__restrict__ m,
     m[k] = mk;
     v[k] = vk;
     p[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
-  }
-}
-
-// Smoothed probe columns: for columns [c0, c1) of the S columns, V <- sc (V -
-// om T) with T = Ahat V (one damped-Jacobi step on the Jacobi-scaled matrix;
-// sc is the column scale, applied once after the last step).
-__global__ void k_smooth_probes(int N, float *__restrict__ V,
-                                const float *__restrict__ T, float om, float sc,
-                                int c0, int c1) {
-  const size_t n = (size_t)N * S;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int c = (int)(i % S);
-    if (c >= c0 && c < c1) V[i] = sc * fmaf(-om, T[i], V[i]);
   }
 }
 
