@@ -31,6 +31,7 @@
 #include "learned.cuh"
 #include "persist.cuh"
 #include "sell.cuh"
+#include "slices.cuh"
 #include "solve64.cuh"
 #include "train.cuh"
 
@@ -180,6 +181,19 @@ struct Band64 {
   int KP = 0;             // the kernel's number of offsets
 };
 
+// Sorted slices of A (slices.cuh) for the persistent plain solve of matrices that
+// do not fit the by-offset form. The pattern is laid out once, the values are
+// filled in once per set of values.
+struct Slices {
+  void *plan = nullptr;  // perm, inv, base
+  void *mem = nullptr;   // col, val, vectors in slot order
+  int *perm = nullptr, *inv = nullptr, *base = nullptr, *col = nullptr;
+  double *val = nullptr;
+  double *vec[5] = {};   // x r q p C
+  int T = 0;             // window: rows of a CTA's step
+  bool planned = false, filled = false, ok = false;
+};
+
 struct cgx_handle {
   int device = 0;
   // Device blocks of replaced matrices, kept for the next upload
@@ -240,6 +254,7 @@ struct cgx_handle {
 
   // Values by offset of the persistent plain solves.
   Band64 b64;
+  Slices sl;
   RedMem *red = nullptr;  // barrier state of the persistent solves (gridred.cuh)
 
   // Scratch: state, partial sums, dot result, validation flag, barrier state.
@@ -358,6 +373,12 @@ static void dev_free(cgx_handle *h, void *p) {
   h->spare.emplace(it->second, p);
 }
 
+static void slices_free(cgx_handle *h, Slices &S) {
+  if (S.plan) dev_free(h, S.plan);
+  if (S.mem) dev_free(h, S.mem);
+  S = Slices{};
+}
+
 static void drop_graphs(cgx_handle *h) {
   for (auto &g : h->graphs) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -395,6 +416,7 @@ static void free_matrix(cgx_handle *h) {
   h->band_tried = false;
   if (h->b64.mem) dev_free(h, h->b64.mem);
   h->b64 = Band64{};
+  slices_free(h, h->sl);
   h->format = -1;
   h->N = h->nz = 0;
   h->ptr = h->index = nullptr;
@@ -1800,6 +1822,11 @@ constexpr int kSolve64SplitMinRows = 1100000;
 // of them on (160^3, 131 MB: 78.3 -> 76.3 us; 128^3, 67 MB: 37.7 -> 36.4;
 // 112^3, 45 MB, which stay in L2: 23.1 -> 24.2).
 constexpr size_t kSolve64PrefetchBytes = (size_t)60 << 20;
+// At most the seven offsets of the 7-point stencil.
+static bool few_offsets(const cgx_handle *h) {
+  return h->b64.planned && !h->b64.all.empty() && (int)h->b64.all.size() <= 7;
+}
+
 // The by-offset values of the current matrix, for a solve in the given loop
 // mode. They are used when they take no more bytes than the entries of the
 // uploaded layout (12 each): a matrix whose offsets are mostly empty stays on
@@ -1813,7 +1840,7 @@ static cgx_status ensure_band64(cgx_handle *h, const Rows &A, int loop, bool *us
     B.half = half_offsets(B.all);
     B.planned = true;
   }
-  if (loop == CGX_LOOP_GRAPH && (int)B.all.size() <= 7 && h->N > kSolve64FusedMaxRows &&
+  if (loop == CGX_LOOP_GRAPH && few_offsets(h) && h->N > kSolve64FusedMaxRows &&
       h->N < kSolve64SplitMinRows)
     return CGX_SUCCESS;
   *use = B.ok;
@@ -1858,15 +1885,46 @@ static cudaError_t launch_coop(cgx_handle *h, const void *kern, int grid, int T,
 // 86.0.)
 constexpr int kSolve64Resident = 192 << 10;
 
+// The same on sorted slices, whose gathers need more of the L1 (slices.cuh).
+constexpr int kSliceResident = 160 << 10;
+
 // The loop of a plain FP64 solve as one cooperative launch, after the set-up
 // kernel. *ran = false when the GPU cannot hold the grid at once (a device
 // shared through MPS limits): the caller then runs the graph.
+template <typename Mat, bool FUSED, int T>
+static cudaError_t launch_solve64_on(cgx_handle *h, const Mat &A, Solve64Args a, bool *ran) {
+  const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+  a.red = h->red;
+  a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
+  // Steps of each vector in shared memory, first those of the vector whose
+  // traffic it saves most: r (24 bytes a row and iteration), then x, C and q
+  // (16 each).
+  int room = (Mat::kPerm ? kSliceResident : kSolve64Resident) / (int)(T * sizeof(double));
+  auto take = [&](bool wanted) {
+    const int n = wanted ? std::min(room, a.steps) : 0;
+    room -= n;
+    return n;
+  };
+  a.nr = take(true);
+  a.nx = take(true);
+  a.nc = take(a.C != nullptr);
+  a.nq = take(true);
+  const size_t smem = sizeof(double) * T * (size_t)(a.nr + a.nx + a.nc + a.nq);
+  CgState *st = h->st;
+  void *args[] = {(void *)&A, &a, &st};
+  const cudaError_t e = launch_coop(h, (const void *)k_solve64<Mat, FUSED, T>, grid, T, smem, args);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    *ran = false;
+    return cudaSuccess;
+  }
+  *ran = e == cudaSuccess;
+  return e;
+}
+
 template <int K, bool SYM, bool FUSED, bool PF, int T>
 static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, bool *ran) {
-  *ran = false;
   const Band64 &B = h->b64;
-  const void *kern = (const void *)k_solve64<K, SYM, FUSED, PF, T>;
-  const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
   Solve64Args a{};
   a.x = h->vec[CGX_VECTOR_X];
   a.r = h->vec[CGX_VECTOR_R];
@@ -1875,44 +1933,19 @@ static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, bool *ran) {
   a.C = jacobi ? h->C : nullptr;
   a.p2 = B.p2;
   a.z = B.z;
-  a.red = h->red;
-  a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
-  // Steps of each vector in shared memory, first those of the vector whose
-  // traffic it saves most: r (24 bytes a row and iteration), then x, C and q
-  // (16 each).
-  int room = kSolve64Resident / (int)(T * sizeof(double));
-  auto take = [&](bool wanted) {
-    const int n = wanted ? std::min(room, a.steps) : 0;
-    room -= n;
-    return n;
-  };
-  a.nr = take(true);
-  a.nx = take(true);
-  a.nc = take(jacobi);
-  a.nq = take(true);
-  const size_t smem = sizeof(double) * T * (size_t)(a.nr + a.nx + a.nc + a.nq);
-  Band64View<K, SYM> A;
-  A.U = B.U;
-  A.ld = B.ld;
-  A.N = h->N;
+  BandMat<K, SYM, PF> A;
+  A.B.U = B.U;
+  A.B.ld = B.ld;
+  A.B.N = h->N;
   const std::vector<int> &D = SYM ? B.half : B.all;
-  for (int k = 0; k < K; k++) A.d[k] = k < (int)D.size() ? D[k] : 0;
-  CgState *st = h->st;
-  void *args[] = {&A, &a, &st};
-  const cudaError_t e = launch_coop(h, kern, grid, T, smem, args);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
-  *ran = e == cudaSuccess;
-  return e;
+  for (int k = 0; k < K; k++) A.B.d[k] = k < (int)D.size() ? D[k] : 0;
+  return launch_solve64_on<BandMat<K, SYM, PF>, FUSED, T>(h, A, a, ran);
 }
 
 // loop: CGX_LOOP_PERSISTENT and CGX_LOOP_PERSISTENT_SPLIT force a form.
 template <int K, bool SYM>
 static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ran) {
   constexpr bool kWide = K > 7;
-  *ran = false;
   if (loop == CGX_LOOP_GRAPH) {
     loop = h->N <= (kWide ? kSolve64FusedMaxRowsWide : kSolve64FusedMaxRows)
                ? CGX_LOOP_PERSISTENT
@@ -1929,6 +1962,7 @@ static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ra
 }
 
 static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ran) {
+  *ran = false;
   if (!h->b64.sym)
     return h->b64.KP == 7 ? launch_solve64<7, false>(h, jacobi, loop, ran)
                           : launch_solve64<kBand64MaxK, false>(h, jacobi, loop, ran);
@@ -1937,6 +1971,127 @@ static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ra
   case 4: return launch_solve64<4, true>(h, jacobi, loop, ran);
   }
   return launch_solve64<kBand64MaxHalf, true>(h, jacobi, loop, ran);
+}
+
+// --- sorted slices -----------------------------------------------------------
+
+// The width of a window and of the solve's CTAs: as many CTAs as SMs where the rows
+// suffice, then as wide as possible.
+static int slices_width(const cgx_handle *h) {
+  return h->N <= h->num_sms * 256 ? 256 : h->N <= h->num_sms * 512 ? 512 : 1024;
+}
+
+// The sorted slices of the current matrix. They are used when they hold at most
+// a quarter more entries than the matrix; *use = false also when the device has
+// no room for them.
+template <typename Rows>
+static cgx_status ensure_slices(cgx_handle *h, const Rows &A, bool *use) {
+  Slices &S = h->sl;
+  *use = false;
+  const int N = h->N, nsl = (N + 31) / 32;
+  cudaStream_t s = h->stream;
+  if (!S.planned) {
+    S.planned = true;
+    S.T = slices_width(h);
+    Carver c;
+    const size_t o_perm = c.take<int>((size_t)N), o_inv = c.take<int>((size_t)N);
+    const size_t o_base = c.take<int>((size_t)nsl + 1);
+    const size_t o_wid = c.take<int>((size_t)nsl);
+    const size_t o_sums = c.take<int>((size_t)nsl / cgx::learned::kScanBlock + 1);
+    cudaError_t e = dev_alloc(h, &S.plan, c.off);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return CGX_SUCCESS;
+    }
+    CUDA_TRY(e);
+    char *b = (char *)S.plan;
+    S.perm = (int *)(b + o_perm);
+    S.inv = (int *)(b + o_inv);
+    S.base = (int *)(b + o_base);
+    CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), s));
+    const int windows = (N + S.T - 1) / S.T;
+    k_slices_sort<<<windows, S.T, 0, s>>>(N, A, std::min(h->num_sms, windows), S.perm, S.inv,
+                                          (int *)(b + o_wid), h->flag);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(scan(h, nsl, (int *)(b + o_wid), S.base, (int *)(b + o_sums)));
+    int flag = 0, total = 0;
+    CUDA_TRY(cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaMemcpyAsync(&total, S.base + nsl, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    const size_t entries = 32 * (size_t)total;
+    bool fits = flag == 0 && 4 * entries <= 5 * (size_t)h->nz;
+    if (fits) {
+      Carver d;
+      const size_t o_col = d.take<int>(entries), o_val = d.take<double>(entries);
+      size_t o_vec[5];
+      for (auto &o : o_vec) o = d.take<double>((size_t)N);
+      e = dev_alloc(h, &S.mem, d.off);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        fits = false;
+      } else {
+        CUDA_TRY(e);
+        char *m = (char *)S.mem;
+        S.col = (int *)(m + o_col);
+        S.val = (double *)(m + o_val);
+        for (int k = 0; k < 5; k++) S.vec[k] = (double *)(m + o_vec[k]);
+      }
+    }
+    if (!fits) {
+      dev_free(h, S.plan);
+      S.plan = nullptr;
+    }
+    S.ok = fits;
+  }
+  if (S.ok && !S.filled) {
+    k_slices_fill<double><<<grid_stream(h, (size_t)N), kThreads, 0, s>>>(
+        N, A, S.perm, S.inv, S.base, S.col, S.val);
+    CUDA_TRY(cudaGetLastError());
+    S.filled = true;
+  }
+  *use = S.ok;
+  return CGX_SUCCESS;
+}
+
+static cudaError_t launch_slices64(cgx_handle *h, bool jacobi, bool *ran) {
+  const Slices &S = h->sl;
+  SliceMat A;
+  A.S = SliceView<double>{S.base, S.col, S.val, h->N};
+  A.perm = S.perm;
+  Solve64Args a{};
+  a.x = S.vec[0];
+  a.r = S.vec[1];
+  a.q = S.vec[2];
+  a.p = S.vec[3];
+  a.C = jacobi ? S.vec[4] : nullptr;
+  a.xo = h->vec[CGX_VECTOR_X];
+  a.ro = h->vec[CGX_VECTOR_R];
+  a.qo = h->vec[CGX_VECTOR_Q];
+  a.po = h->vec[CGX_VECTOR_P];
+  a.Co = h->C;
+  *ran = false;
+  switch (S.T) {
+  case 256: return launch_solve64_on<SliceMat, false, 256>(h, A, a, ran);
+  case 512: return launch_solve64_on<SliceMat, false, 512>(h, A, a, ran);
+  }
+  return launch_solve64_on<SliceMat, false, 1024>(h, A, a, ran);
+}
+
+// The persistent plain solve of the matrix given by its rows, if it has a form
+// for it.
+template <typename Rows>
+static cgx_status solve_persistent64(cgx_handle *h, const Rows &A, const cgx_options &o,
+                                     bool jacobi, bool *ran) {
+  bool band = false, slices = false;
+  CGX_TRY(ensure_band64(h, A, o.loop, &band));
+  // A matrix of few offsets that its own rule leaves to the graph stays there.
+  if (!band && !h->b64.ok && !few_offsets(h)) CGX_TRY(ensure_slices(h, A, &slices));
+  if (!band && !slices) return CGX_SUCCESS;
+  reset_host_state(h, o.max_iterations, o.tolerance, false, 0);
+  CGX_TRY(push_state(h));
+  CUDA_TRY(launch_pcg_setup(h, jacobi));
+  CUDA_TRY(band ? launch_solve64(h, jacobi, o.loop, ran) : launch_slices64(h, jacobi, ran));
+  return CGX_SUCCESS;
 }
 
 static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
@@ -1952,19 +2107,12 @@ static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
   const int loop = want_persist ? CGX_LOOP_GRAPH : o.loop;
   bool ran = false;
   if (want_persist) {
-    bool use = false;
     CUDA_TRY(cudaEventRecord(h->ev[0], s));
     if (h->format == CGX_FORMAT_ELL)
-      CGX_TRY(ensure_band64(h, RowsEll{h->ell_length, h->ell_index, h->ell_data, h->ell_width},
-                            o.loop, &use));
+      CGX_TRY(solve_persistent64(
+          h, RowsEll{h->ell_length, h->ell_index, h->ell_data, h->ell_width}, o, jacobi, &ran));
     else
-      CGX_TRY(ensure_band64(h, RowsCrs{h->ptr, h->index, h->value}, o.loop, &use));
-    if (use) {
-      reset_host_state(h, o.max_iterations, o.tolerance, false, 0);
-      CGX_TRY(push_state(h));
-      CUDA_TRY(launch_pcg_setup(h, jacobi));
-      CUDA_TRY(launch_solve64(h, jacobi, o.loop, &ran));
-    }
+      CGX_TRY(solve_persistent64(h, RowsCrs{h->ptr, h->index, h->value}, o, jacobi, &ran));
     if (ran) {
       CUDA_TRY(cudaEventRecord(h->ev[1], s));
       CGX_TRY(pull_state(h));
@@ -1976,7 +2124,7 @@ static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
 
   if (ran) {
     // done
-  } else   if (loop == CGX_LOOP_GRAPH) {
+  } else if (loop == CGX_LOOP_GRAPH) {
     GraphEntry *ge = nullptr;
     const int key = 100 + (jacobi ? 1 : 0);
     CGX_TRY(build_while_graph(
@@ -3092,6 +3240,7 @@ cgx_status cgx_update_crs_values(cgx_handle *h, const double *value) {
   h->f32_valid = false;
   h->c_valid = false;
   h->b64.filled = h->b64.ok = false;
+  h->sl.filled = false;
   if (h->L) h->L->has_factor = false;
   return CGX_SUCCESS;
 }

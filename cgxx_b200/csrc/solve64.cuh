@@ -1,9 +1,10 @@
-// Persistent FP64 solves on matrices of few column offsets.
+// Persistent FP64 solves.
 //
-// A whole plain FP64 PCG loop is one cooperative launch when A's rows are
-// sorted and its entries lie on few diagonals (structured-grid stencils). What
-// this buys against the graph of k_crs, k_pcg_update and k_pcg_direction:
-//  - bytes: the CRS product reads 12 bytes per nonzero (84 per row of the
+// A whole plain FP64 PCG loop is one cooperative launch: on A by offset when its
+// rows are sorted and its entries lie on few diagonals (structured-grid stencils),
+// else on A in sorted slices (slices.cuh). What this buys against the graph of
+// k_crs, k_pcg_update and k_pcg_direction:
+//  - bytes (by offset): the CRS product reads 12 bytes per nonzero (84 per row of the
 //    7-point matrix). The values are stored by offset (U_k is an array over
 //    the rows) without indices: 8 bytes per offset and row, and if A is
 //    symmetric, only the diagonal and the upper offsets (32 bytes per row); a
@@ -45,6 +46,7 @@
 
 #include "band.cuh"
 #include "gridred.cuh"
+#include "slices.cuh"
 
 namespace cgx {
 
@@ -188,11 +190,39 @@ __device__ __forceinline__ void band64_prefetch(const Band64View<K, SYM> &B, int
 
 // --- the solve ---------------------------------------------------------------
 
+// The matrix of a solve. kPerm: the solve's rows are slots of the sorted slices,
+// and the vectors are brought into their order and back.
+template <int K, bool SYM, bool PF>
+struct BandMat {
+  static constexpr bool kPerm = false;
+  Band64View<K, SYM> B;
+  __device__ int n() const { return B.N; }
+  __device__ int from(int i) const { return i; }
+  __device__ void prefetch(int i, int stride) const {
+    if (PF) band64_prefetch(B, i, stride);
+  }
+  template <typename XAt>
+  __device__ double row(int i, XAt xat) const {
+    return band64_row(B, i, xat);
+  }
+};
+struct SliceMat {
+  static constexpr bool kPerm = true;
+  SliceView<double> S;
+  const int *perm;
+  __device__ int n() const { return S.N; }
+  __device__ int from(int i) const { return __ldg(perm + i); }
+};
+
 struct Solve64Args {
   double *x, *r, *q;
   const double *C;  // NULL: no preconditioner (z = r)
   double *p;        // the direction; fused: in turn with p2
   double *p2, *z;   // fused only
+  // kPerm: the same vectors in the matrix's own row order, read at the start and
+  // written at the end (x, r, q, C and p above are then in slot order).
+  double *xo, *ro, *qo, *po;
+  const double *Co;
   RedMem *red;              // barrier state, its counter 0 at launch
   int steps;                // rows per thread
   int nr, nx, nc, nq;       // steps of r, x, C, q held in shared memory
@@ -205,16 +235,17 @@ __device__ __forceinline__ double *vec_at(double *sm, int n, double *g, int k, i
   return k < n ? sm + (k * TPB + (int)threadIdx.x) : g + i;
 }
 
-template <int K, bool SYM, bool FUSED, bool PF, int TPB>
-__global__ void __launch_bounds__(TPB, 1)
-    k_solve64(Band64View<K, SYM> A, Solve64Args a, CgState *st) {
+template <typename Mat, bool FUSED, int TPB>
+__global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgState *st) {
+  constexpr bool PERM = Mat::kPerm;
+  static_assert(!(PERM && FUSED), "the fused form is the band's");
   extern __shared__ __align__(16) double sm[];
   __shared__ double sc[8];  // scalars of the last grid sum
   double *const sr = sm;
   double *const sx = sr + (size_t)a.nr * TPB;
   double *const scd = sx + (size_t)a.nx * TPB;
   double *const sq = scd + (size_t)a.nc * TPB;
-  const int N = A.N, steps = a.steps;
+  const int N = A.n(), steps = a.steps;
   const int i0 = blockIdx.x * TPB + threadIdx.x, stride = gridDim.x * TPB;
   const double nrm0 = st->nrm0, tol = st->tol;
   const int maxit = st->max_iter;
@@ -224,13 +255,22 @@ __global__ void __launch_bounds__(TPB, 1)
   bool ok = true;
 
   for (int k = 0, i = i0; k < steps && i < N; k++, i += stride) {
-    if (k < a.nr) sr[k * TPB + threadIdx.x] = a.r[i];
-    if (k < a.nx) sx[k * TPB + threadIdx.x] = a.x[i];
-    if (k < a.nc) scd[k * TPB + threadIdx.x] = a.C ? a.C[i] : 1.0;
+    if constexpr (PERM) {
+      const int j = A.from(i);
+      *vec_at<TPB>(sr, a.nr, a.r, k, i) = a.ro[j];
+      *vec_at<TPB>(sx, a.nx, a.x, k, i) = a.xo[j];
+      if (a.C) *vec_at<TPB>(scd, a.nc, const_cast<double *>(a.C), k, i) = a.Co[j];
+      a.p[i] = a.po[j];
+    } else {
+      if (k < a.nr) sr[k * TPB + threadIdx.x] = a.r[i];
+      if (k < a.nx) sx[k * TPB + threadIdx.x] = a.x[i];
+      if (k < a.nc) scd[k * TPB + threadIdx.x] = a.C ? a.C[i] : 1.0;
+    }
   }
+  if (PERM) ok = grid_barrier<TPB>(a.red, round);  // p is read across CTAs
   // C of step k: shared, global, or 1 (1 * r is r, exactly).
   auto c_at = [&](int k, int i) {
-    return k < a.nc ? scd[k * TPB + threadIdx.x] : a.C ? __ldg(a.C + i) : 1.0;
+    return k < a.nc ? scd[k * TPB + threadIdx.x] : a.C ? __ldca(a.C + i) : 1.0;
   };
   // f(tag, k, i) over this thread's rows, two steps per call while there are
   // two, so that the loads of both are issued before the first store.
@@ -245,14 +285,14 @@ __global__ void __launch_bounds__(TPB, 1)
   // direction it writes.
   const double *zc = a.p, *po = a.p;
   double *pn = a.p2;
-  for (;;) {
+  while (ok) {
     // A
     double s1[1] = {0.0};
     if constexpr (FUSED) {
       for (int k = 0, i = i0; k < steps && i < N; k++, i += stride) {
         const double poi = __ldca(po + i), pi = madd(__ldca(zc + i), beta, poi);
-        const double qi = band64_row(
-            A, i, [&](int j) { return madd(__ldca(zc + j), beta, __ldca(po + j)); });
+        const double qi =
+            A.row(i, [&](int j) { return madd(__ldca(zc + j), beta, __ldca(po + j)); });
         double *xp = vec_at<TPB>(sx, a.nx, a.x, k, i);
         *xp = madd(*xp, alpha, poi);
         pn[i] = pi;
@@ -261,12 +301,19 @@ __global__ void __launch_bounds__(TPB, 1)
       }
     } else {
       const double *p = a.p;
-      for (int k = 0, i = i0; k < steps && i < N; k++, i += stride) {
-        if (PF) band64_prefetch(A, i, stride);
-        const double pi = __ldca(p + i);
-        const double qi = band64_row(A, i, [&](int j) { return __ldca(p + j); });
+      auto x_at = [&](int j) { return __ldca(p + j); };
+      auto put = [&](int k, int i, double pi, double qi) {
         *vec_at<TPB>(sq, a.nq, a.q, k, i) = qi;
         s1[0] = fma(pi, qi, s1[0]);
+      };
+      if constexpr (PERM) {
+        slice_rows<TPB, kSliceInFlight>(A.S, steps, x_at, put);
+      } else {
+        for (int k = 0, i = i0; k < steps && i < N; k++, i += stride) {
+          A.prefetch(i, stride);
+          const double pi = __ldca(p + i);
+          put(k, i, pi, A.row(i, x_at));
+        }
       }
     }
     ok = grid_sum<TPB, 1>(a.red, round, s1, sc, [&](const double (&s)[1], double *o) {
@@ -357,9 +404,17 @@ __global__ void __launch_bounds__(TPB, 1)
       *xp = madd(*xp, alpha, pi);
       if (po != a.p) a.p[i] = pi;
     }
-    if (k < a.nx) a.x[i] = *xp;
-    if (k < a.nr) a.r[i] = sr[k * TPB + threadIdx.x];
-    if (k < a.nq) a.q[i] = sq[k * TPB + threadIdx.x];
+    if constexpr (PERM) {
+      const int j = A.from(i);
+      a.xo[j] = *xp;
+      a.ro[j] = *vec_at<TPB>(sr, a.nr, a.r, k, i);
+      a.qo[j] = *vec_at<TPB>(sq, a.nq, a.q, k, i);
+      a.po[j] = a.p[i];
+    } else {
+      if (k < a.nx) a.x[i] = *xp;
+      if (k < a.nr) a.r[i] = sr[k * TPB + threadIdx.x];
+      if (k < a.nq) a.q[i] = sq[k * TPB + threadIdx.x];
+    }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->r2 = sc[5];

@@ -1,0 +1,97 @@
+"""Persistent FP64 solves on sorted slices (slices.cuh) against the chunked loop of
+the CRS kernels, on matrices that no by-offset form holds. A row's products are
+added in the same order, so q = A p of the first iteration is bit-identical; the
+dot products' order differs, so later iterates agree to rounding: the solutions at
+a residual of 1e-11 differ by at most 1e-11 times the condition number, which is
+below 1e2 for these diagonally dominant matrices (1e-8 with a margin of 10).
+"""
+import numpy as np
+import pytest
+
+import cgxx_b200 as cg
+from cgxx_b200 import generators as G
+from conftest import random_crs
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense_row(N, extra, seed):
+    """random_crs plus a symmetric first row and column of `extra` entries."""
+    A = random_crs(N, 0, 8, seed=seed, spd=True)
+    rows = np.repeat(np.arange(N), np.diff(A.ptr))
+    j = np.arange(1, extra + 1)
+    d = np.zeros(N)
+    d[0], d[1:extra + 1] = 0.01 * extra, 0.01
+    rows = np.concatenate([rows, np.zeros(extra, int), j, np.arange(N)])
+    cols = np.concatenate([A.index, j, np.zeros(extra, int), np.arange(N)])
+    vals = np.concatenate([A.value, np.full(2 * extra, -0.01), d + 1e-3])
+    key = rows.astype(np.int64) * N + cols
+    uk, inv = np.unique(key, return_inverse=True)
+    return G.crs_from_unsorted(N, uk // N, uk % N, np.bincount(inv, weights=vals))
+
+
+def _shuffled(A, seed):
+    """The same matrix, each row's entries in another order."""
+    rng = np.random.default_rng(seed)
+    index, value = A.index.copy(), A.value.copy()
+    for i in range(A.N):
+        s = slice(A.ptr[i], A.ptr[i + 1])
+        o = rng.permutation(A.ptr[i + 1] - A.ptr[i])
+        index[s], value[s] = index[s][o], value[s][o]
+    return G.Crs(A.N, A.ptr, index, value)
+
+
+CASES = [
+    ("random_33", lambda: random_crs(33, 0, 12, seed=1, spd=True)),
+    ("random_255", lambda: random_crs(255, 0, 20, seed=2, spd=True)),
+    ("random_1500", lambda: random_crs(1500, 0, 40, seed=3, spd=True)),
+    ("shuffled_3000", lambda: _shuffled(random_crs(3000, 0, 20, seed=4, spd=True), 5)),
+    ("graph_40001", lambda: G.geometric_graph(40001, seed=6)),   # 512-thread CTAs
+    ("graph_160001", lambda: G.geometric_graph(160001, seed=7)),  # 1024, two steps
+    ("dense_row_2000", lambda: _dense_row(2000, 1500, 8)),
+    ("row_of_5000", lambda: _dense_row(6000, 5000, 9)),  # too long: stays on the graph
+]
+
+
+@pytest.mark.parametrize("fmt", ["crs", "coo"])
+@pytest.mark.parametrize("name,make", CASES, ids=[c[0] for c in CASES])
+def test_solve_matches_the_chunked_loop(name, make, fmt):
+    A = make()
+    rng = np.random.default_rng(10)
+    k = rng.standard_normal(A.N)
+    x0 = rng.standard_normal(A.N)
+    jac = name != "random_255"
+    pc = cg.PRECOND_JACOBI if jac else cg.PRECOND_NONE
+    with cg.Handle(0) as h:
+        if fmt == "crs":
+            h.upload_crs(A.ptr, A.index, A.value)
+        else:
+            h.upload_coo(A.N, np.repeat(np.arange(A.N), np.diff(A.ptr)).astype(np.int32), A.index,
+                         A.value)
+        h.jacobi_from_matrix()
+        h.set_vector("K", k)
+
+        def solve(loop, **kw):
+            h.set_vector("X", x0)
+            r = h.solve(loop=loop, preconditioner=pc, **kw)
+            return r, {v: h.get_vector(v) for v in "XRPQ"}
+
+        _, one = solve(cg.LOOP_GRAPH, max_iterations=1, tolerance=1e-300)
+        _, ref1 = solve(cg.LOOP_CHUNKED, max_iterations=1, tolerance=1e-300)
+        assert np.array_equal(one["Q"], ref1["Q"])
+        for v in "XRP":
+            assert np.allclose(one[v], ref1[v], rtol=0, atol=1e-13 * np.abs(ref1[v]).max())
+        a, va = solve(cg.LOOP_GRAPH, max_iterations=2000, tolerance=1e-11)
+        b, vb = solve(cg.LOOP_CHUNKED, max_iterations=2000, tolerance=1e-11)
+        assert a["converged"] and b["converged"]
+        assert abs(a["iterations"] - b["iterations"]) <= 1 + 0.02 * b["iterations"]
+        # Graphs (shift 1e-3) are worse conditioned than the random matrices.
+        bound = 1e-5 if name.startswith("graph") else 1e-8
+        assert np.linalg.norm(va["X"] - vb["X"]) <= bound * np.linalg.norm(vb["X"])
+        # New values of the same pattern reach the slices.
+        if fmt == "crs":
+            h.update_crs_values(2.0 * A.value)
+            h.jacobi_from_matrix()
+            c, vc = solve(cg.LOOP_GRAPH, max_iterations=2000, tolerance=1e-11)
+            assert c["converged"]
+            assert np.linalg.norm(2.0 * vc["X"] - vb["X"]) <= bound * np.linalg.norm(vb["X"])
