@@ -29,6 +29,7 @@
 #include "ingest.cuh"
 #include "kernels.cuh"
 #include "learned.cuh"
+#include "offsets.cuh"
 #include "persist.cuh"
 #include "sell.cuh"
 #include "slices.cuh"
@@ -194,6 +195,16 @@ struct Slices {
   bool planned = false, filled = false, ok = false;
 };
 
+// FP32 values of a symmetric A by offset (offsets.cuh), for the persistent inner
+// solves of matrices with 5 to 14 non-negative offsets. Planned once per pattern,
+// filled with the FP32 copy.
+struct Off32 {
+  float *U = nullptr;  // kBand64MaxHalf arrays of ld rows
+  size_t ld = 0;
+  std::vector<int> half;
+  bool planned = false, ok = false;
+};
+
 struct cgx_handle {
   int device = 0;
   // Device blocks of replaced matrices, kept for the next upload
@@ -251,6 +262,7 @@ struct cgx_handle {
   // Symmetric band copy, preferred over SELL-U when A fits it.
   Band band;
   bool band_tried = false;
+  Off32 off32;
 
   // Values by offset of the persistent plain solves.
   Band64 b64;
@@ -417,6 +429,8 @@ static void free_matrix(cgx_handle *h) {
   if (h->b64.mem) dev_free(h, h->b64.mem);
   h->b64 = Band64{};
   slices_free(h, h->sl);
+  if (h->off32.U) dev_free(h, h->off32.U);
+  h->off32 = Off32{};
   h->format = -1;
   h->N = h->nz = 0;
   h->ptr = h->index = nullptr;
@@ -1723,12 +1737,11 @@ static cgx_status band_plan(cgx_handle *h, Band &B) {
   return CGX_SUCCESS;
 }
 
-// U from A's current values by the offsets D; *fits: the rows ascend and, for
-// SYM, the values are symmetric.
-template <bool SYM, typename Rows>
-static cgx_status band64_fill(cgx_handle *h, const Rows &A, const std::vector<int> &D,
-                              bool *fits) {
-  Band64 &B = h->b64;
+// U (KP arrays of ld rows) from A's current values by the offsets D; *fits: the
+// rows ascend and, for SYM, the values are symmetric.
+template <bool SYM, typename VT, typename Rows>
+static cgx_status band64_fill(cgx_handle *h, const Rows &A, const std::vector<int> &D, VT *U,
+                              int KP, size_t ld, bool *fits) {
   const int N = h->N;
   Band64Offsets o{};
   o.K = (int)D.size();
@@ -1737,15 +1750,15 @@ static cgx_status band64_fill(cgx_handle *h, const Rows &A, const std::vector<in
   CUDA_TRY(dev_alloc(h, (void **)&counts, 2 * sizeof(unsigned long long)));
   unsigned long long hc[2] = {0, 0};
   int flag = 0;
-  cudaError_t e = cudaMemsetAsync(B.U, 0, sizeof(double) * B.KP * B.ld, h->stream);
+  cudaError_t e = cudaMemsetAsync(U, 0, sizeof(VT) * KP * ld, h->stream);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(counts, 0, 2 * sizeof(unsigned long long), h->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream);
   if (e == cudaSuccess) {
-    k_band64_fill<SYM><<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, o, B.U, B.ld,
-                                                                      counts, h->flag);
+    k_band64_fill<SYM><<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, o, U, ld, counts,
+                                                                      h->flag);
     if (SYM)
-      k_band64_check<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, o, B.U, B.ld, counts,
+      k_band64_check<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, A, o, U, ld, counts,
                                                                     h->flag);
     e = cudaGetLastError();
   }
@@ -1853,12 +1866,12 @@ static cgx_status ensure_band64(cgx_handle *h, const Rows &A, int loop, bool *us
   const int KA = na <= 7 ? 7 : kBand64MaxK;
   if (nh > 0 && nh <= kBand64MaxHalf && dense(KH)) {
     CGX_TRY(band64_alloc(h, KH, &got));
-    if (got) CGX_TRY(band64_fill<true>(h, A, B.half, &fits));
+    if (got) CGX_TRY(band64_fill<true>(h, A, B.half, B.U, B.KP, B.ld, &fits));
     B.sym = fits;
   }
   if (!fits && na > 0 && na <= kBand64MaxK && dense(KA)) {
     CGX_TRY(band64_alloc(h, KA, &got));
-    if (got) CGX_TRY(band64_fill<false>(h, A, B.all, &fits));
+    if (got) CGX_TRY(band64_fill<false>(h, A, B.all, B.U, B.KP, B.ld, &fits));
   }
   if (!fits && B.mem) {
     dev_free(h, B.mem);
@@ -2246,6 +2259,39 @@ static cgx_status band_fill(cgx_handle *h, Band &B) {
   return CGX_SUCCESS;
 }
 
+// A's FP32 values by offset, where A is symmetric with at most 14 non-negative
+// offsets and dense on them: 4 bytes an offset against 6 an entry of the 16-bit
+// CRS copy. Without room on the device the solves run as if it did not fit.
+static cgx_status fill_off32(cgx_handle *h) {
+  Off32 &B = h->off32;
+  const RowsCrs A{h->ptr, h->index, h->value};
+  B.ok = false;
+  if (!B.planned) {
+    B.planned = true;
+    std::vector<int> all;
+    CGX_TRY(band_offsets(h, A, all));
+    B.half = half_offsets(all);
+    B.ld = round_up((size_t)h->N, 32);
+  }
+  if (B.half.empty() || (int)B.half.size() > kBand64MaxHalf ||
+      4.0 * kBand64MaxHalf * h->N > 6.0 * h->nz)
+    return CGX_SUCCESS;
+  if (!B.U) {
+    const cudaError_t e = dev_alloc(h, (void **)&B.U, sizeof(float) * kBand64MaxHalf * B.ld);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return CGX_SUCCESS;
+    }
+    CUDA_TRY(e);
+  }
+  CGX_TRY(band64_fill<true>(h, A, B.half, B.U, kBand64MaxHalf, B.ld, &B.ok));
+  if (!B.ok) {
+    dev_free(h, B.U);
+    B.U = nullptr;
+  }
+  return CGX_SUCCESS;
+}
+
 static cgx_status ensure_f32(cgx_handle *h) {
   if (h->f32_valid) return CGX_SUCCESS;
   const int N = h->N;
@@ -2314,6 +2360,7 @@ static cgx_status ensure_f32(cgx_handle *h) {
         (size_t)h->nz, h->sa.map, h->value, h->sa_val);
     CUDA_TRY(cudaGetLastError());
   }
+  if (!h->band.ok) CGX_TRY(fill_off32(h));
   CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
   k_delta16<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, h->ptr, h->index,
                                                            h->idx16, h->flag);
@@ -2404,7 +2451,7 @@ constexpr int kInnerFusedMaxRows[2] = {1000000, 2300000};  // Jacobi, learned
 constexpr int kInnerNarrowCtaRows = 148 * 256;  // 256-thread CTAs up to here
 constexpr int kInnerWideCtaRows = 200000;       // learned: 1024 from here on
 constexpr int kInnerPrefetchMinRows = 3000000;
-// SELL-U: 512-thread CTAs up to two passes of them, 1024 beyond (27-point grids,
+// SELL-U and by offset: 512-thread CTAs up to two passes of them, 1024 beyond (27-point grids,
 // Jacobi / learned: 24^3 9.2 / 15.7 against 11.9 / 20.8 us per iteration, 48^3
 // 10.0 / 20.2 against 12.4 / 23.3, 64^3 15.2 / 30.6 against 13.8 / 25.0, 96^3
 // 32.1 / 69.8 against 27.0 / 51.9).
@@ -2482,6 +2529,19 @@ static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
   a.C = h->C32;
   a.eps = LEARNED ? h->L->eps : 0.f;
   a.red = h->red;
+  if (form == InnerForm::kSell && !LEARNED && h->off32.ok) {
+    Band64View<kBand64MaxHalf, true, float> B;
+    B.U = h->off32.U;
+    B.ld = h->off32.ld;
+    B.N = h->N;
+    for (int k = 0; k < kBand64MaxHalf; k++)
+      B.d[k] = k < (int)h->off32.half.size() ? h->off32.half[k] : 0;
+    if (h->N <= kInnerSellNarrowRows)
+      return launch_inner_split<OffsetPhases<kBand64MaxHalf, 512>, 512>(
+          h, OffsetPhases<kBand64MaxHalf, 512>{B}, a);
+    return launch_inner_split<OffsetPhases<kBand64MaxHalf, 1024>, 1024>(
+        h, OffsetPhases<kBand64MaxHalf, 1024>{B}, a);
+  }
   if (form == InnerForm::kSell) {
     const SellUView<float> A{h->sa.meta, h->sa.off, h->sa_val, h->N};
     SellUView<__nv_bfloat16> G{}, GT{};
@@ -2521,6 +2581,7 @@ static cudaError_t launch_inner_persist(cgx_handle *h, bool learned, InnerForm f
 // same.
 static bool sell_fits(const cgx_handle *h, bool learned) {
   const long long slices = ((long long)h->N + 31) / 32;
+  if (!learned && !h->band.ok && h->off32.ok) return true;
   if (h->band.ok || !h->sa.ok || !h->sa_val || h->sa.uniform != slices)
     return false;
   if (!learned) return true;

@@ -57,6 +57,7 @@
 #include "band.cuh"
 #include "gridred.cuh"
 #include "kernels.cuh"
+#include "offsets.cuh"
 #include "sell.cuh"
 
 namespace cgx {
@@ -342,6 +343,69 @@ struct BandPhases {
     });
     return s;
   }
+};
+
+// Row i of a symmetric A stored by offset (lower values from the mirror rows)
+// times x, in ascending column order; x is finite, so an entry that a row does
+// not have (value 0) adds nothing. The loads of a group of slots are issued
+// before its sums.
+template <int K, typename X>
+__device__ __forceinline__ float offset_row(const Band64View<K, true, float> &B, int i, const X &x) {
+  const float *__restrict__ U = B.U;
+  const unsigned nmax = (unsigned)(B.N - 1);
+  constexpr int kSlots = 2 * K - 1, G = 7;
+  float sum = 0.f;
+#pragma unroll
+  for (int s0 = 0; s0 < kSlots; s0 += G) {
+    float v[G], xv[G];
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+      const int s = s0 + g;
+      if (s >= kSlots) continue;
+      if (s < K - 1) {
+        const int k = K - 1 - s, j = i - B.d[k], jc = max(j, 0);
+        v[g] = __ldg(U + k * B.ld + jc);
+        xv[g] = x(jc);
+        v[g] = j < 0 ? 0.f : v[g];
+      } else {
+        const int k = s - (K - 1);
+        v[g] = __ldg(U + k * B.ld + i);
+        xv[g] = x((int)min((unsigned)(i + B.d[k]), nmax));
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < G; g++)
+      if (s0 + g < kSlots) sum = fmaf(v[g], xv[g], sum);
+  }
+  return sum;
+}
+
+// A by offset (Jacobi only): half the value bytes of the uniform slices. Bound by
+// L2's throughput, as the mirror values of the plane below come from there: at
+// 128^3 about 108 bytes a row and product, 226 MB in 36 us. us per iteration of
+// 27-point grids, uniform slices -> by offset: 24^3 10.9 -> 7.3, 48^3 14.2 -> 8.7,
+// 64^3 15.8 -> 11.4, 96^3 28.6 -> 20.1, 128^3 55.2 -> 44.0. (Groups of 7, 9 or 14
+// slots, L2 prefetch of the next step's values, 128 or 160 KB of resident vectors:
+// within 1 us.)
+template <int K, int TPB>
+struct OffsetPhases {
+  static constexpr bool kLearned = false;
+  static constexpr bool kTiled = true;
+  Band64View<K, true, float> A;
+  __device__ int N() const { return A.N; }
+  __device__ double q_rows(const InnerArgs &a, float *sq) const {
+    double s = 0.0;
+    const float *p = a.p;
+    const int stride = gridDim.x * TPB;
+    for (int k = 0, i = blockIdx.x * TPB + threadIdx.x; k < a.steps && i < A.N; k++, i += stride) {
+      const float pv = ldv(p + i), qv = offset_row(A, i, Stored{p});
+      *tile_at<TPB>(sq, a.nq, a.q, k, threadIdx.x, i) = qv;
+      s = fma((double)pv, (double)qv, s);
+    }
+    return s;
+  }
+  __device__ void y_rows(const InnerArgs &) const {}
+  __device__ double z_rows(const InnerArgs &, float *, float *) const { return 0.0; }
 };
 
 // SELL-U: A, G and G^T in uniform slices (sell.cuh). Its products deal slices,
