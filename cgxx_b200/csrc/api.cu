@@ -182,17 +182,29 @@ struct Band64 {
   int KP = 0;             // the kernel's number of offsets
 };
 
-// Sorted slices of A (slices.cuh) for the persistent plain solve of matrices that
-// do not fit the by-offset form. The pattern is laid out once, the values are
-// filled in once per set of values.
+// One matrix in sorted slices (slices.cuh): the pattern is laid out once, the values
+// are filled in once per set of values.
+template <typename VT>
+struct SliceArrays {
+  void *plan = nullptr, *mem = nullptr;
+  int *base = nullptr, *col = nullptr;
+  VT *val = nullptr;
+  bool planned = false, ok = false, filled = false;
+};
+
+// The slot order of a handle's matrix and what is stored in it: A for the
+// persistent plain and inner solves of matrices without a form by offset, and the
+// learned factor. The vectors serve one launch at a time.
 struct Slices {
-  void *plan = nullptr;  // perm, inv, base
-  void *mem = nullptr;   // col, val, vectors in slot order
-  int *perm = nullptr, *inv = nullptr, *base = nullptr, *col = nullptr;
-  double *val = nullptr;
-  double *vec[5] = {};   // x r q p C
-  int T = 0;             // window: rows of a CTA's step
-  bool planned = false, filled = false, ok = false;
+  void *mem = nullptr, *vec_mem = nullptr;
+  int *perm = nullptr, *inv = nullptr;
+  double *vec = nullptr;  // five FP64 or ten FP32 vectors, `ld` rows of FP64 each
+  size_t ld = 0;
+  int T = 0;              // window: rows of a CTA's step
+  bool planned = false, ok = false;
+  SliceArrays<double> a64;
+  SliceArrays<float> a32;
+  SliceArrays<__nv_bfloat16> g, gt;
 };
 
 // FP32 values of a symmetric A by offset (offsets.cuh), for the persistent inner
@@ -385,9 +397,20 @@ static void dev_free(cgx_handle *h, void *p) {
   h->spare.emplace(it->second, p);
 }
 
+template <typename VT>
+static void slices_free(cgx_handle *h, SliceArrays<VT> &S) {
+  dev_free(h, S.plan);
+  dev_free(h, S.mem);
+  S = SliceArrays<VT>{};
+}
+
 static void slices_free(cgx_handle *h, Slices &S) {
-  if (S.plan) dev_free(h, S.plan);
-  if (S.mem) dev_free(h, S.mem);
+  slices_free(h, S.a64);
+  slices_free(h, S.a32);
+  slices_free(h, S.g);
+  slices_free(h, S.gt);
+  dev_free(h, S.mem);
+  dev_free(h, S.vec_mem);
   S = Slices{};
 }
 
@@ -1994,89 +2017,112 @@ static int slices_width(const cgx_handle *h) {
   return h->N <= h->num_sms * 256 ? 256 : h->N <= h->num_sms * 512 ? 512 : 1024;
 }
 
-// The sorted slices of the current matrix. They are used when they hold at most
-// a quarter more entries than the matrix; *use = false also when the device has
-// no room for them.
+// A block for the slices: *p stays NULL when the device has no room for it.
+static cgx_status slices_alloc(cgx_handle *h, void **p, size_t bytes) {
+  const cudaError_t e = dev_alloc(h, p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return CGX_SUCCESS;
+  }
+  CUDA_TRY(e);
+  return CGX_SUCCESS;
+}
+
+// The slot order of the current matrix; h->sl.ok if there is one (no row is too
+// long, and there is room).
 template <typename Rows>
-static cgx_status ensure_slices(cgx_handle *h, const Rows &A, bool *use) {
+static cgx_status ensure_slots(cgx_handle *h, const Rows &A) {
   Slices &S = h->sl;
-  *use = false;
-  const int N = h->N, nsl = (N + 31) / 32;
+  if (S.planned) return CGX_SUCCESS;
+  S.planned = true;
+  const int N = h->N;
+  S.T = slices_width(h);
+  S.ld = round_up((size_t)N, 32);
+  Carver c;
+  const size_t o_perm = c.take<int>((size_t)N), o_inv = c.take<int>((size_t)N);
+  const size_t o_wid = c.take<int>((size_t)(N + 31) / 32);
+  CGX_TRY(slices_alloc(h, &S.mem, c.off));
+  CGX_TRY(slices_alloc(h, &S.vec_mem, 5 * sizeof(double) * S.ld));
+  if (!S.mem || !S.vec_mem) return CGX_SUCCESS;
+  S.perm = (int *)((char *)S.mem + o_perm);
+  S.inv = (int *)((char *)S.mem + o_inv);
+  S.vec = (double *)S.vec_mem;
+  CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
+  const int windows = (N + S.T - 1) / S.T;
+  k_slices_sort<<<windows, S.T, 0, h->stream>>>(N, A, std::min(h->num_sms, windows), S.perm,
+                                                S.inv, (int *)((char *)S.mem + o_wid), h->flag);
+  CUDA_TRY(cudaGetLastError());
+  int flag = 0;
+  CUDA_TRY(cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CUDA_TRY(cudaStreamSynchronize(h->stream));
+  S.ok = flag == 0;
+  return CGX_SUCCESS;
+}
+
+// The rows A (nnz entries) in sorted slices, with their current values; M.ok if
+// they hold at most `most` times the entries and there is room.
+template <typename VT, typename Rows>
+static cgx_status slices_matrix(cgx_handle *h, const Rows &A, size_t nnz, double most,
+                                SliceArrays<VT> &M) {
+  const Slices &S = h->sl;
+  const int N = h->N, nsl = (N + 31) / 32, grid = grid_stream(h, (size_t)N);
   cudaStream_t s = h->stream;
-  if (!S.planned) {
-    S.planned = true;
-    S.T = slices_width(h);
+  if (!M.planned) {
+    M.planned = true;
     Carver c;
-    const size_t o_perm = c.take<int>((size_t)N), o_inv = c.take<int>((size_t)N);
-    const size_t o_base = c.take<int>((size_t)nsl + 1);
-    const size_t o_wid = c.take<int>((size_t)nsl);
+    const size_t o_base = c.take<int>((size_t)nsl + 1), o_wid = c.take<int>((size_t)nsl);
     const size_t o_sums = c.take<int>((size_t)nsl / cgx::learned::kScanBlock + 1);
-    cudaError_t e = dev_alloc(h, &S.plan, c.off);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      return CGX_SUCCESS;
-    }
-    CUDA_TRY(e);
-    char *b = (char *)S.plan;
-    S.perm = (int *)(b + o_perm);
-    S.inv = (int *)(b + o_inv);
-    S.base = (int *)(b + o_base);
-    CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), s));
-    const int windows = (N + S.T - 1) / S.T;
-    k_slices_sort<<<windows, S.T, 0, s>>>(N, A, std::min(h->num_sms, windows), S.perm, S.inv,
-                                          (int *)(b + o_wid), h->flag);
+    CGX_TRY(slices_alloc(h, &M.plan, c.off));
+    if (!M.plan) return CGX_SUCCESS;
+    char *b = (char *)M.plan;
+    M.base = (int *)(b + o_base);
+    k_slices_width<<<grid, kThreads, 0, s>>>(N, A, S.perm, (int *)(b + o_wid));
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(scan(h, nsl, (int *)(b + o_wid), S.base, (int *)(b + o_sums)));
-    int flag = 0, total = 0;
-    CUDA_TRY(cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaMemcpyAsync(&total, S.base + nsl, sizeof(int), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(scan(h, nsl, (int *)(b + o_wid), M.base, (int *)(b + o_sums)));
+    int total = 0;
+    CUDA_TRY(cudaMemcpyAsync(&total, M.base + nsl, sizeof(int), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
     const size_t entries = 32 * (size_t)total;
-    bool fits = flag == 0 && 4 * entries <= 5 * (size_t)h->nz;
-    if (fits) {
-      Carver d;
-      const size_t o_col = d.take<int>(entries), o_val = d.take<double>(entries);
-      size_t o_vec[5];
-      for (auto &o : o_vec) o = d.take<double>((size_t)N);
-      e = dev_alloc(h, &S.mem, d.off);
-      if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        fits = false;
-      } else {
-        CUDA_TRY(e);
-        char *m = (char *)S.mem;
-        S.col = (int *)(m + o_col);
-        S.val = (double *)(m + o_val);
-        for (int k = 0; k < 5; k++) S.vec[k] = (double *)(m + o_vec[k]);
-      }
-    }
-    if (!fits) {
-      dev_free(h, S.plan);
-      S.plan = nullptr;
-    }
-    S.ok = fits;
+    if ((double)entries > most * (double)nnz) return CGX_SUCCESS;
+    Carver d;
+    const size_t o_col = d.take<int>(entries), o_val = d.take<VT>(entries);
+    CGX_TRY(slices_alloc(h, &M.mem, d.off));
+    if (!M.mem) return CGX_SUCCESS;
+    M.col = (int *)((char *)M.mem + o_col);
+    M.val = (VT *)((char *)M.mem + o_val);
+    M.ok = true;
   }
-  if (S.ok && !S.filled) {
-    k_slices_fill<double><<<grid_stream(h, (size_t)N), kThreads, 0, s>>>(
-        N, A, S.perm, S.inv, S.base, S.col, S.val);
+  if (M.ok && !M.filled) {
+    k_slices_fill<VT><<<grid, kThreads, 0, s>>>(N, A, S.perm, S.inv, M.base, M.col, M.val);
     CUDA_TRY(cudaGetLastError());
-    S.filled = true;
+    M.filled = true;
   }
-  *use = S.ok;
+  return CGX_SUCCESS;
+}
+
+// Padding that the slices of A, and of the factor, may add.
+constexpr double kSlicesMost = 1.25, kSlicesMostFactor = 2.0;
+
+// FP64 slices of the current matrix; *use = false if it does not fit them.
+template <typename Rows>
+static cgx_status ensure_slices(cgx_handle *h, const Rows &A, bool *use) {
+  CGX_TRY(ensure_slots(h, A));
+  if (h->sl.ok) CGX_TRY(slices_matrix(h, A, (size_t)h->nz, kSlicesMost, h->sl.a64));
+  *use = h->sl.a64.ok;
   return CGX_SUCCESS;
 }
 
 static cudaError_t launch_slices64(cgx_handle *h, bool jacobi, bool *ran) {
   const Slices &S = h->sl;
   SliceMat A;
-  A.S = SliceView<double>{S.base, S.col, S.val, h->N};
+  A.S = SliceView<double>{S.a64.base, S.a64.col, S.a64.val, h->N};
   A.perm = S.perm;
   Solve64Args a{};
-  a.x = S.vec[0];
-  a.r = S.vec[1];
-  a.q = S.vec[2];
-  a.p = S.vec[3];
-  a.C = jacobi ? S.vec[4] : nullptr;
+  a.x = S.vec;
+  a.r = S.vec + S.ld;
+  a.q = S.vec + 2 * S.ld;
+  a.p = S.vec + 3 * S.ld;
+  a.C = jacobi ? S.vec + 4 * S.ld : nullptr;
   a.xo = h->vec[CGX_VECTOR_X];
   a.ro = h->vec[CGX_VECTOR_R];
   a.qo = h->vec[CGX_VECTOR_Q];
@@ -2459,13 +2505,13 @@ constexpr int kInnerSellNarrowRows = 148 * 1024;
 
 // One inner solve as a persistent cooperative launch (persist.cuh), after
 // the path's start kernel(s): one CTA per SM, and no more CTAs than tiles.
-enum class InnerForm { kGraph, kFused, kSplit, kSell };
+enum class InnerForm { kGraph, kFused, kSplit, kSell, kSlices };
 
 template <typename Phases, int T>
 static cudaError_t launch_inner_split(cgx_handle *h, const Phases &P, InnerArgs a) {
   const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
   a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
-  int room = kInnerResident / (int)(T * sizeof(float));
+  int room = (Phases::kPerm ? kSliceResident : kInnerResident) / (int)(T * sizeof(float));
   auto take = [&](bool wanted) {
     const int n = wanted ? std::min(room, a.steps) : 0;
     room -= n;
@@ -2555,6 +2601,38 @@ static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
     return launch_inner_split<SellPhases<LEARNED, 1024>, 1024>(
         h, SellPhases<LEARNED, 1024>{A, G, GT}, a);
   }
+  if (form == InnerForm::kSlices) {
+    const Slices &S = h->sl;
+    // Slot order: ten FP32 vectors.
+    float *v = (float *)S.vec;
+    a.ro = a.r;
+    a.po = a.p;
+    a.Co = a.C;
+    a.dout = a.d;
+    a.r = v;
+    a.p = v + S.ld;
+    a.C = v + 2 * S.ld;
+    a.d = v + 3 * S.ld;
+    a.q = v + 4 * S.ld;
+    a.z = v + 5 * S.ld;
+    a.y = v + 6 * S.ld;
+    const SliceView<float> A{S.a32.base, S.a32.col, S.a32.val, h->N};
+    SliceView<__nv_bfloat16> G{}, GT{};
+    if (LEARNED) {
+      G = SliceView<__nv_bfloat16>{S.g.base, S.g.col, S.g.val, h->N};
+      GT = SliceView<__nv_bfloat16>{S.gt.base, S.gt.col, S.gt.val, h->N};
+    }
+    switch (S.T) {
+    case 256:
+      return launch_inner_split<SlicePhases<LEARNED, 256>, 256>(
+          h, SlicePhases<LEARNED, 256>{A, G, GT, S.perm}, a);
+    case 512:
+      return launch_inner_split<SlicePhases<LEARNED, 512>, 512>(
+          h, SlicePhases<LEARNED, 512>{A, G, GT, S.perm}, a);
+    }
+    return launch_inner_split<SlicePhases<LEARNED, 1024>, 1024>(
+        h, SlicePhases<LEARNED, 1024>{A, G, GT, S.perm}, a);
+  }
   const BandView<4> A = band_view(h);
   GBandView G{};
   if (LEARNED) G = gband_view(h);
@@ -2606,6 +2684,28 @@ static bool persist_fits(const cgx_handle *h, bool learned) {
 // kInnerFusedMaxRows rows) or split (larger ones). CGX_LOOP_PERSISTENT and
 // CGX_LOOP_PERSISTENT_SPLIT force their form on the band; the default
 // CGX_LOOP_GRAPH takes the persistent form that measured fastest.
+// The sorted slices of an irregular matrix (neither a band nor uniform slices) and,
+// for the learned path, of its factor; *use if they fit.
+static cgx_status ensure_inner_slices(cgx_handle *h, bool want_learned, bool *use) {
+  *use = false;
+  Slices &S = h->sl;
+  Learned *L = h->L;
+  if (h->band.ok || h->off32.ok || h->sa.ok || (want_learned && (L->gb_ok || !L->sell_ok)))
+    return CGX_SUCCESS;
+  const RowsCrs A{h->ptr, h->index, h->value};
+  CGX_TRY(ensure_slots(h, A));
+  if (!S.ok) return CGX_SUCCESS;
+  CGX_TRY(slices_matrix(h, A, (size_t)h->nz, kSlicesMost, S.a32));
+  if (want_learned && S.a32.ok) {
+    const learned::RowsFactor<false> G{L->gptr, L->gcol, nullptr, L->ghat, L->dis};
+    const learned::RowsFactor<true> GT{L->tptr, L->tcol, L->t2g, L->ghat, L->dis};
+    CGX_TRY(slices_matrix(h, G, (size_t)L->nnzL, kSlicesMostFactor, S.g));
+    CGX_TRY(slices_matrix(h, GT, (size_t)L->nnzL, kSlicesMostFactor, S.gt));
+  }
+  *use = S.a32.ok && (!want_learned || (S.g.ok && S.gt.ok));
+  return CGX_SUCCESS;
+}
+
 static InnerForm inner_form(const cgx_handle *h, const cgx_options &o, bool learned) {
   if (sell_fits(h, learned) &&
       (o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT_SPLIT))
@@ -2673,7 +2773,13 @@ static cgx_status solve_mixed(cgx_handle *h, const cgx_options &o,
 
   // The persistent inner solves (persist.cuh); the fused form's start also
   // stores z.
-  const InnerForm form = inner_form(h, o, want_learned);
+  InnerForm form = inner_form(h, o, want_learned);
+  if (form == InnerForm::kGraph &&
+      (o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT_SPLIT)) {
+    bool slices = false;
+    CGX_TRY(ensure_inner_slices(h, want_learned, &slices));
+    if (slices) form = InnerForm::kSlices;
+  }
   const bool persist = form != InnerForm::kGraph;
   // PERSISTENT on a matrix without the band form runs as GRAPH.
   const bool graph_loop =
@@ -2869,7 +2975,7 @@ static cgx_status solve_mixed(cgx_handle *h, const cgx_options &o,
   res.spmv_launches = res.update_launches = res.direction_launches = launches;
   res.inner_form = form == InnerForm::kFused ? 1
                    : form == InnerForm::kSplit ? 2
-                   : form == InnerForm::kSell  ? 3
+                   : form == InnerForm::kSell || form == InnerForm::kSlices ? 3
                                                : 0;
   res.inner_launches = inner_launches;
   res.inner_ms = t_inner;
@@ -3301,7 +3407,7 @@ cgx_status cgx_update_crs_values(cgx_handle *h, const double *value) {
   h->f32_valid = false;
   h->c_valid = false;
   h->b64.filled = h->b64.ok = false;
-  h->sl.filled = false;
+  h->sl.a64.filled = h->sl.a32.filled = false;
   if (h->L) h->L->has_factor = false;
   return CGX_SUCCESS;
 }
@@ -3441,6 +3547,7 @@ cgx_status cgx_learned_factor(cgx_handle *h, cgx_gnn *gn, double eps) {
   if (!(eps >= 0)) return fail(CGX_ERROR_INVALID_ARGUMENT, "eps must be >= 0");
   DeviceGuard guard(h->device);
   CUDA_TRY(gnn_forward(h, gn->params, true));
+  h->sl.g.filled = h->sl.gt.filled = false;
   // eps is a kernel argument of the captured inner-solve graphs: a new value
   // needs new graphs (the factor's values are in device memory and need none).
   if (h->L->eps != (float)eps) drop_graphs(h);

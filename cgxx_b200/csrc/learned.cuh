@@ -477,6 +477,22 @@ __global__ void k_assemble(int nnzL, const int *__restrict__ grow,
   }
 }
 
+// Rows of G (TRANS: of G^T, over G's entries t2g) for the sorted slices, with the
+// values that k_assemble gives the other BF16 copies.
+template <bool TRANS>
+struct RowsFactor {
+  const int *ptr, *idx, *t2g;
+  const float *ghat;
+  const double *dis;
+  __device__ int begin(int i) const { return ptr[i]; }
+  __device__ int end(int i) const { return ptr[i + 1]; }
+  __device__ int col(int, int j) const { return idx[j]; }
+  __device__ float val(int i, int j) const {
+    return TRANS ? (float)(dis[idx[j]] * (double)ghat[t2g[j]])
+                 : (float)(dis[i] * (double)ghat[j]);
+  }
+};
+
 // ---------------------------------------------------------------------------
 // Training: Adam, probes (the loss and its gradient: train.cuh)
 

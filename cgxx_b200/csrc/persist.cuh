@@ -59,6 +59,7 @@
 #include "kernels.cuh"
 #include "offsets.cuh"
 #include "sell.cuh"
+#include "slices.cuh"
 
 namespace cgx {
 
@@ -101,6 +102,10 @@ struct InnerArgs {
   int rows;        // fused: rows per CTA
   int below;       // fused learned: CTAs below whose y phase C reads
   int nz, nr, nd, nq, nc;  // tiles or passes held in shared memory
+  // Sorted slices: r, p, C and d in the matrix's own row order; the vectors above
+  // are in slot order.
+  const float *ro, *po, *Co;
+  float *dout;
 };
 
 // Scalars of the loop, shared by a CTA's threads: sc[0] alpha, sc[1] residual,
@@ -271,6 +276,7 @@ struct BandPhases {
   // q (and z) of a tile may be kept in shared memory: the thread that writes
   // row i of a product is the tile's, so the tile stays in its CTA.
   static constexpr bool kTiled = true;
+  static constexpr bool kPerm = false;
   BandView<4> A;
   GBandView G;
   __device__ int N() const { return A.N; }
@@ -391,6 +397,7 @@ template <int K, int TPB>
 struct OffsetPhases {
   static constexpr bool kLearned = false;
   static constexpr bool kTiled = true;
+  static constexpr bool kPerm = false;
   Band64View<K, true, float> A;
   __device__ int N() const { return A.N; }
   __device__ double q_rows(const InnerArgs &a, float *sq) const {
@@ -414,6 +421,7 @@ template <bool LEARNED, int TPB>
 struct SellPhases {
   static constexpr bool kLearned = LEARNED;
   static constexpr bool kTiled = false;
+  static constexpr bool kPerm = false;
   static constexpr int U = 8;
   SellUView<float> A;
   SellUView<__nv_bfloat16> G, GT;
@@ -463,6 +471,46 @@ struct SellPhases {
   }
 };
 
+// Sorted slices (slices.cuh), for irregular matrices: a slot's rows of all the
+// products belong to the same tile.
+template <bool LEARNED, int TPB>
+struct SlicePhases {
+  static constexpr bool kLearned = LEARNED;
+  static constexpr bool kTiled = true;
+  static constexpr bool kPerm = true;
+  SliceView<float> A;
+  SliceView<__nv_bfloat16> G, GT;
+  const int *perm;
+  __device__ int N() const { return A.N; }
+  __device__ double q_rows(const InnerArgs &a, float *sq) const {
+    double s = 0.0;
+    slice_rows<TPB, kSliceInFlight32>(
+        A, a.steps, [&](int j) { return ldv(a.p + j); },
+        [&](int k, int i, float pv, float qv) {
+          *tile_at<TPB>(sq, a.nq, a.q, k, threadIdx.x, i) = qv;
+          s = fma((double)pv, (double)qv, s);
+        });
+    return s;
+  }
+  __device__ void y_rows(const InnerArgs &a) const {
+    slice_rows<TPB, kSliceInFlight32>(
+        GT, a.steps, [&](int j) { return ldv(a.r + j); },
+        [&](int, int i, float, float yv) { a.y[i] = yv; });
+  }
+  __device__ double z_rows(const InnerArgs &a, float *sz, float *sr) const {
+    double s = 0.0;
+    slice_rows<TPB, kSliceInFlight32>(
+        G, a.steps, [&](int j) { return ldv(a.y + j); },
+        [&](int k, int i, float, float gy) {
+          const float rv = *tile_at<TPB>(sr, a.nr, a.r, k, threadIdx.x, i);
+          const float zv = fmaf(a.eps * ldv(a.C + i), rv, gy);
+          *tile_at<TPB>(sz, a.nz, a.z, k, threadIdx.x, i) = zv;
+          s = fma((double)rv, (double)zv, s);
+        });
+    return s;
+  }
+};
+
 template <typename Phases, int TPB>
 __global__ void __launch_bounds__(TPB, 1)
     k_inner_split(Phases P, InnerArgs a, CgState *st) {
@@ -487,12 +535,33 @@ __global__ void __launch_bounds__(TPB, 1)
       if (i < N) sm[k * TPB + threadIdx.x] = g[i];
     }
   };
-  bring(sr, a.nr, a.r);
-  bring(sd, a.nd, a.d);
-  bring(scd, a.nc, a.C);
-  __syncthreads();
+  if constexpr (Phases::kPerm) {
+    for (int k = 0; k < steps; k++) {
+      const long long l = ((long long)k * gridDim.x + blockIdx.x) * TPB + threadIdx.x;
+      if (l >= N) break;
+      const int i = (int)l, j = __ldg(P.perm + i), t = threadIdx.x;
+      *tile_at<TPB>(sr, a.nr, a.r, k, t, i) = a.ro[j];
+      *tile_at<TPB>(sd, a.nd, a.d, k, t, i) = 0.f;
+      *tile_at<TPB>(scd, a.nc, const_cast<float *>(a.C), k, t, i) = a.Co[j];
+      a.p[i] = a.po[j];
+    }
+    ok = grid_barrier<TPB>(a.red, round);  // p is read across CTAs
+  } else {
+    bring(sr, a.nr, a.r);
+    bring(sd, a.nd, a.d);
+    bring(scd, a.nc, a.C);
+    __syncthreads();
+  }
+  // C is written in this launch only with kPerm (then not the read-only path).
+  auto cval = [&](int k, int o, int i) {
+    return !Phases::kPerm ? __ldg(a.C + i) : k < a.nc ? scd[k * TPB + o] : ldv(a.C + i);
+  };
+  auto c4 = [&](int i) {
+    const float4 *c = reinterpret_cast<const float4 *>(a.C + i);
+    return Phases::kPerm ? *c : __ldg(c);
+  };
 
-  for (;;) {
+  while (ok) {
     // A
     {
       const double s[1] = {P.q_rows(a, sq)};
@@ -513,7 +582,7 @@ __global__ void __launch_bounds__(TPB, 1)
             const float4 r0 = quad(rp), qv = quad(tile_at<TPB>(sq, a.nq, a.q, k, o, i));
             const float4 cv = LEARNED ? r0
                               : k < a.nc ? quad(scd + (k * TPB + o))
-                                         : __ldg(reinterpret_cast<const float4 *>(a.C + i));
+                                         : c4(i);
             const float4 rv = fma4(na, qv, r0);
             quad_to(rp, rv);
             if (LEARNED && k < a.nr) quad_to(a.r + i, rv);
@@ -526,7 +595,7 @@ __global__ void __launch_bounds__(TPB, 1)
             *rp = rv;
             if (LEARNED && k < a.nr) a.r[i] = rv;
             s[0] = fma((double)rv, (double)rv, s[0]);
-            if (!LEARNED) s[1] = fma((double)rv, (double)(__ldg(a.C + i) * rv), s[1]);
+            if (!LEARNED) s[1] = fma((double)rv, (double)(cval(k, o, i) * rv), s[1]);
           });
       if (LEARNED) {
         const double s1[1] = {s[0]};
@@ -570,8 +639,7 @@ __global__ void __launch_bounds__(TPB, 1)
               zv = quad(tile_at<TPB>(sz, a.nz, a.z, k, o, i));
             } else {
               const float4 rv = quad(tile_at<TPB>(sr, a.nr, a.r, k, o, i));
-              const float4 cv = k < a.nc ? quad(scd + (k * TPB + o))
-                                         : __ldg(reinterpret_cast<const float4 *>(a.C + i));
+              const float4 cv = k < a.nc ? quad(scd + (k * TPB + o)) : c4(i);
               zv = mul4(cv, rv);
             }
             quad_to(dp, fma4(al, pv, dv));
@@ -581,7 +649,7 @@ __global__ void __launch_bounds__(TPB, 1)
             float *dp = tile_at<TPB>(sd, a.nd, a.d, k, o, i);
             const float pi = ldv(a.p + i);
             const float zi = LEARNED ? *tile_at<TPB>(sz, a.nz, a.z, k, o, i)
-                                     : __ldg(a.C + i) * *tile_at<TPB>(sr, a.nr, a.r, k, o, i);
+                                     : cval(k, o, i) * *tile_at<TPB>(sr, a.nr, a.r, k, o, i);
             *dp = fmaf(al, pi, *dp);
             if (!stop) a.p[i] = fmaf(be, pi, zi);
           });
@@ -590,9 +658,17 @@ __global__ void __launch_bounds__(TPB, 1)
   }
   // d is what the refinement step needs.
   __syncthreads();
-  for (int k = 0; k < a.nd; k++) {
-    const long long i = ((long long)k * gridDim.x + blockIdx.x) * TPB + threadIdx.x;
-    if (i < N) a.d[i] = sd[k * TPB + threadIdx.x];
+  if constexpr (Phases::kPerm) {
+    for (int k = 0; k < steps; k++) {
+      const long long l = ((long long)k * gridDim.x + blockIdx.x) * TPB + threadIdx.x;
+      if (l >= N) break;
+      a.dout[__ldg(P.perm + (int)l)] = *tile_at<TPB>(sd, a.nd, a.d, k, threadIdx.x, (int)l);
+    }
+  } else {
+    for (int k = 0; k < a.nd; k++) {
+      const long long i = ((long long)k * gridDim.x + blockIdx.x) * TPB + threadIdx.x;
+      if (i < N) a.d[i] = sd[k * TPB + threadIdx.x];
+    }
   }
   loop.publish(st, sc, alpha, beta, ok);
 }

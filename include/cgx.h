@@ -141,7 +141,8 @@ typedef struct cgx_result {
   int inner_form;        /* MIXED: how the inner solves ran: 0 per-iteration
                             kernels, 1 fused persistent launches, 2 split
                             persistent launches on the band form, 3 split
-                            persistent launches on SELL-U (cgx_loop) */
+                            persistent launches on SELL-U, values by offset or
+                            sorted slices (cgx_loop) */
   int inner_launches;    /* MIXED, inner_form 1 or 2: persistent launches */
   double inner_ms;       /* MIXED, inner_form 1 or 2: their device time (CUDA
                             events around each launch) */

@@ -10,6 +10,7 @@ import pytest
 
 import cgxx_b200 as cg
 from cgxx_b200 import generators as G
+from cgxx_b200 import learned as LRN
 from conftest import random_crs
 
 pytestmark = pytest.mark.gpu
@@ -95,3 +96,41 @@ def test_solve_matches_the_chunked_loop(name, make, fmt):
             c, vc = solve(cg.LOOP_GRAPH, max_iterations=2000, tolerance=1e-11)
             assert c["converged"]
             assert np.linalg.norm(2.0 * vc["X"] - vb["X"]) <= bound * np.linalg.norm(vb["X"])
+
+
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("name,make", CASES[:7], ids=[c[0] for c in CASES[:7]])
+def test_inner_solves_match_the_kernels(name, make, learned):
+    """Mixed solves on the FP32 and BF16 slices against the loop of per-iteration
+    kernels (CRS and SELL-U): the same products in the same order, so the inner
+    counts agree to 2 % + 2 and both reach the FP64 residual. The second solve is
+    on new values with a new factor."""
+    A = make()
+    rng = np.random.default_rng(12)
+    k = A.matvec(rng.uniform(-1, 1, A.N))
+    tol = 1e-10
+    with cg.Handle(0) as h:
+        h.upload_crs(A.ptr, A.index, A.value)
+        net = cg.Gnn(0, LRN.load_weights(LRN.DEFAULT_WEIGHTS)[0])
+        for scale in (1.0, 2.0):
+            h.update_crs_values(scale * A.value)
+            h.jacobi_from_matrix()
+            pc = cg.PRECOND_JACOBI
+            if learned:
+                h.learned_setup()
+                h.learned_factor(net, 1e-4)
+                pc = cg.PRECOND_LEARNED
+            h.set_vector("K", scale * k)
+            its = {}
+            for loop in (cg.LOOP_GRAPH, cg.LOOP_KERNELS):
+                h.fill_vector("X", 0.0)
+                r = h.solve(max_iterations=20000, tolerance=tol, loop=loop, preconditioner=pc,
+                            precision=cg.PRECISION_MIXED)
+                assert r["converged"] and r["fell_back"] == 0
+                if loop == cg.LOOP_GRAPH and name in ("graph_40001", "graph_160001"):
+                    assert r["inner_form"] == 3
+                x = h.get_vector("X")
+                assert np.linalg.norm(k - A.matvec(x)) <= tol * np.linalg.norm(k)
+                its[loop] = r["iterations"]
+            assert abs(its[cg.LOOP_GRAPH] - its[cg.LOOP_KERNELS]) <= 0.02 * its[cg.LOOP_KERNELS] + 2
+        net.close()
