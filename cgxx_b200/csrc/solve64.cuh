@@ -155,7 +155,7 @@ __device__ __forceinline__ double *vec_at(double *sm, int n, double *g, int k, i
   return k < n ? sm + (k * TPB + (int)threadIdx.x) : g + i;
 }
 
-template <typename Mat, bool FUSED, int TPB>
+template <typename Mat, bool FUSED, bool CLUSTER, int TPB>
 __global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgState *st) {
   constexpr bool PERM = Mat::kPerm;
   static_assert(!(PERM && FUSED), "the fused form is the band's");
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgStat
       if (k < a.nc) scd[k * TPB + threadIdx.x] = a.C ? a.C[i] : 1.0;
     }
   }
-  if (PERM) ok = grid_barrier<TPB>(a.red, round);  // p is read across CTAs
+  if (PERM) ok = sync_over<CLUSTER, TPB>(a.red, round);  // p is read across CTAs
   // C of step k: shared, global, or 1 (1 * r is r, exactly).
   auto c_at = [&](int k, int i) {
     return k < a.nc ? scd[k * TPB + threadIdx.x] : a.C ? __ldca(a.C + i) : 1.0;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgStat
         }
       }
     }
-    ok = grid_sum<TPB, 1>(a.red, round, s1, sc, [&](const double (&s)[1], double *o) {
+    ok = sum_over<CLUSTER, TPB, 1>(a.red, round, s1, sc, [&](const double (&s)[1], double *o) {
       o[0] = rho / s[0];
       o[1] = s[0];
     });
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgStat
       }
     });
     it++;
-    ok = grid_sum<TPB, 2>(a.red, round, s2, sc + 2, [&](const double (&s)[2], double *o) {
+    ok = sum_over<CLUSTER, TPB, 2>(a.red, round, s2, sc + 2, [&](const double (&s)[2], double *o) {
       o[0] = sqrt(s[0]) / nrm0;
       o[1] = s[1] / rho;
       o[2] = s[1];
@@ -312,10 +312,11 @@ __global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgStat
           if (!stop) a.p[i + u * stride] = madd(__dmul_rn(cv[u], rv[u]), beta, pv[u]);
         }
       });
-      if (stop || !(ok = grid_barrier<TPB>(a.red, round))) break;
+      if (stop || !(ok = sync_over<CLUSTER, TPB>(a.red, round))) break;
     }
   }
 
+  if (CLUSTER) cluster_sync();
   // Back to the global vectors; fused: the last x update and p.
   for (int k = 0, i = i0; k < steps && i < N; k++, i += stride) {
     double *xp = vec_at<TPB>(sx, a.nx, a.x, k, i);
