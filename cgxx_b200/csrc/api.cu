@@ -214,7 +214,7 @@ struct Off32 {
   float *U = nullptr;  // kBand64MaxHalf arrays of ld rows
   size_t ld = 0;
   std::vector<int> half;
-  bool planned = false, ok = false;
+  bool planned = false, filled = false, ok = false;
 };
 
 struct cgx_handle {
@@ -2378,10 +2378,11 @@ static cgx_status band_fill(cgx_handle *h, Band &B) {
 // A's FP32 values by offset, where A is symmetric with at most 14 non-negative
 // offsets and dense on them: 4 bytes an offset against 6 an entry of the 16-bit
 // CRS copy. Without room on the device the solves run as if it did not fit.
-static cgx_status fill_off32(cgx_handle *h) {
+static cgx_status ensure_off32(cgx_handle *h) {
   Off32 &B = h->off32;
+  if (B.filled || h->band.ok) return CGX_SUCCESS;
   const RowsCrs A{h->ptr, h->index, h->value};
-  B.ok = false;
+  B.filled = true;
   if (!B.planned) {
     B.planned = true;
     std::vector<int> all;
@@ -2476,7 +2477,7 @@ static cgx_status ensure_f32(cgx_handle *h) {
         (size_t)h->nz, h->sa.map, h->value, h->sa_val);
     CUDA_TRY(cudaGetLastError());
   }
-  if (!h->band.ok) CGX_TRY(fill_off32(h));
+  h->off32.filled = h->off32.ok = false;
   CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
   k_delta16<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, h->ptr, h->index,
                                                            h->idx16, h->flag);
@@ -2646,6 +2647,16 @@ static cudaError_t launch_inner_fused(cgx_handle *h, BandView<4> A, GBandView G,
                                h->st);
 }
 
+static Band64View<kBand64MaxHalf, true, float> off32_view(const cgx_handle *h) {
+  Band64View<kBand64MaxHalf, true, float> B;
+  B.U = h->off32.U;
+  B.ld = h->off32.ld;
+  B.N = h->N;
+  for (int k = 0; k < kBand64MaxHalf; k++)
+    B.d[k] = k < (int)h->off32.half.size() ? h->off32.half[k] : 0;
+  return B;
+}
+
 template <bool LEARNED>
 static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
   InnerArgs a{};
@@ -2661,12 +2672,7 @@ static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
   a.eps = LEARNED ? h->L->eps : 0.f;
   a.red = h->red;
   if (form == InnerForm::kSell && !LEARNED && h->off32.ok) {
-    Band64View<kBand64MaxHalf, true, float> B;
-    B.U = h->off32.U;
-    B.ld = h->off32.ld;
-    B.N = h->N;
-    for (int k = 0; k < kBand64MaxHalf; k++)
-      B.d[k] = k < (int)h->off32.half.size() ? h->off32.half[k] : 0;
+    const auto B = off32_view(h);
     if (h->N <= kInnerSellNarrowRows)
       return launch_inner_split<OffsetPhases<kBand64MaxHalf, 512>, 512>(
           h, OffsetPhases<kBand64MaxHalf, 512>{B}, a);
@@ -2675,16 +2681,28 @@ static cudaError_t launch_inner_persist(cgx_handle *h, InnerForm form) {
   }
   if (form == InnerForm::kSell) {
     const SellUView<float> A{h->sa.meta, h->sa.off, h->sa_val, h->N};
-    SellUView<__nv_bfloat16> G{}, GT{};
-    if (LEARNED) {
-      G = SellUView<__nv_bfloat16>{h->L->sg.meta, h->L->sg.off, h->L->sg_val, h->N};
-      GT = SellUView<__nv_bfloat16>{h->L->st.meta, h->L->st.off, h->L->st_val, h->N};
+    if constexpr (LEARNED) {
+      const SellUView<__nv_bfloat16> G{h->L->sg.meta, h->L->sg.off, h->L->sg_val, h->N};
+      const SellUView<__nv_bfloat16> GT{h->L->st.meta, h->L->st.off, h->L->st_val, h->N};
+      if (h->off32.ok) {
+        const auto B = off32_view(h);
+        if (h->N <= kInnerSellNarrowRows)
+          return launch_inner_split<SellPhases<true, true, 512>, 512>(
+              h, SellPhases<true, true, 512>{A, G, GT, B}, a);
+        return launch_inner_split<SellPhases<true, true, 1024>, 1024>(
+            h, SellPhases<true, true, 1024>{A, G, GT, B}, a);
+      }
+      if (h->N <= kInnerSellNarrowRows)
+        return launch_inner_split<SellPhases<true, false, 512>, 512>(
+            h, SellPhases<true, false, 512>{A, G, GT, {}}, a);
+      return launch_inner_split<SellPhases<true, false, 1024>, 1024>(
+          h, SellPhases<true, false, 1024>{A, G, GT, {}}, a);
     }
     if (h->N <= kInnerSellNarrowRows)
-      return launch_inner_split<SellPhases<LEARNED, 512>, 512>(
-          h, SellPhases<LEARNED, 512>{A, G, GT}, a);
-    return launch_inner_split<SellPhases<LEARNED, 1024>, 1024>(
-        h, SellPhases<LEARNED, 1024>{A, G, GT}, a);
+      return launch_inner_split<SellPhases<false, false, 512>, 512>(
+          h, SellPhases<false, false, 512>{A, {}, {}, {}}, a);
+    return launch_inner_split<SellPhases<false, false, 1024>, 1024>(
+        h, SellPhases<false, false, 1024>{A, {}, {}, {}}, a);
   }
   if (form == InnerForm::kSlices) {
     const Slices &S = h->sl;
@@ -2871,9 +2889,10 @@ static cgx_status solve_mixed(cgx_handle *h, const cgx_options &o,
 
   // The persistent inner solves (persist.cuh); the fused form's start also
   // stores z.
+  const bool split = o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT_SPLIT;
+  if (split) CGX_TRY(ensure_off32(h));
   InnerForm form = inner_form(h, o, want_learned);
-  if (form == InnerForm::kGraph &&
-      (o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT_SPLIT)) {
+  if (form == InnerForm::kGraph && split) {
     bool slices = false;
     CGX_TRY(ensure_inner_slices(h, want_learned, &slices));
     if (slices) form = InnerForm::kSlices;

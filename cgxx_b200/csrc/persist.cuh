@@ -417,7 +417,8 @@ struct OffsetPhases {
 
 // SELL-U: A, G and G^T in uniform slices (sell.cuh). Its products deal slices,
 // not tiles, to the warps, so q, z and the r they read are global.
-template <bool LEARNED, int TPB>
+// AOFF: A by offset, whose product deals rows in tiles.
+template <bool LEARNED, bool AOFF, int TPB>
 struct SellPhases {
   static constexpr bool kLearned = LEARNED;
   static constexpr bool kTiled = false;
@@ -425,6 +426,7 @@ struct SellPhases {
   static constexpr int U = 8;
   SellUView<float> A;
   SellUView<__nv_bfloat16> G, GT;
+  Band64View<kBand64MaxHalf, true, float> AO;
   struct OpQ {  // q = A p, <p,q>
     using Acc = Acc1;
     struct Pre {
@@ -455,6 +457,7 @@ struct SellPhases {
   };
   __device__ int N() const { return A.N; }
   __device__ double q_rows(const InnerArgs &a, float *) const {
+    if constexpr (AOFF) return OffsetPhases<kBand64MaxHalf, TPB>{AO}.q_rows(a, nullptr);
     Acc1 acc;
     sellu_rows<float, U, true, TPB>(A, a.p, GatherWeak{}, OpQ{a.p, a.q}, acc);
     return acc.a0;
