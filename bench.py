@@ -363,11 +363,11 @@ def persist_roofline(args, results, N, peak, peak_kind):
 
 
 def plain_persistent(args, N):
-    """Whether the plain solve's loop is one persistent launch: the grids in
-    the default loop, but for the 7-point ones of 0.7M to 1.1M rows
+    """Whether the plain solve's loop is one persistent launch: the default
+    loop's on every workload here, but for the 7-point grids of 0.7M to 1.1M rows
     (kSolve64FusedMaxRows, kSolve64SplitMinRows)."""
-    return not args.graph and args.loop in ("graph", "persistent", "split") and not (
-        args.loop == "graph" and args.stencil == 7 and 700000 < N < 1100000)
+    return args.loop in ("graph", "persistent", "split") and (bool(args.graph) or not (
+        args.loop == "graph" and args.stencil == 7 and 700000 < N < 1100000))
 
 
 def peaks():
@@ -636,7 +636,7 @@ def our_arm(args, world, rank, local):
     # Per solve: the fill of x, the dot of ||b||, a true-residual product per
     # refinement check (outer + 1), and per refinement step its start, the
     # inner solve and the update of x; the learned path adds its set-up
-    # (2 kernels), inference (6) and the start's apply (2 per step).
+    # (2 kernels), inference (5) and the start's apply (2 per step).
     if args.path == "plain" and plain_persistent(args, N):
         per_solve = 3                               # fill, set-up, one launch
     elif args.path == "plain":
@@ -646,7 +646,7 @@ def our_arm(args, world, rank, local):
         per_solve = 2 + (outer + 1) + 2 * outer + inner
     else:
         inner = outer if persist else 6 * iters     # one launch, or 5 kernels + guard
-        per_solve = 2 + 8 + (outer + 1) + 4 * outer + inner
+        per_solve = 2 + 7 + (outer + 1) + 4 * outer + inner
     launches = args.steps * per_solve
 
     cpu = None

@@ -256,7 +256,7 @@ struct cgx_handle {
   // (compact16): the mixed and learned paths read 6 instead of 8 bytes per
   // FP32 entry.
   int16_t *idx16 = nullptr;
-  bool compact16 = false;
+  bool compact16 = false, idx16_tried = false;
   float *d32 = nullptr, *r32 = nullptr, *p32 = nullptr, *q32 = nullptr;
   // Second buffers of the ping-pong pairs (p, r) and z of the persistent
   // inner solves (persist.cuh).
@@ -468,7 +468,7 @@ static void free_matrix(cgx_handle *h) {
   h->p32b = h->r32b = h->z32 = nullptr;
   h->r64 = nullptr;
   h->idx16 = nullptr;
-  h->compact16 = false;
+  h->compact16 = h->idx16_tried = false;
   h->f32_valid = false;
 }
 
@@ -2440,9 +2440,6 @@ static cgx_status ensure_f32(cgx_handle *h) {
     h->r64 = (double *)(base + o_r64);
     h->idx16 = (int16_t *)(base + o_i16);
   }
-  k_to_f32<<<grid_stream(h, h->nz), kThreads, 0, h->stream>>>(
-      (size_t)h->nz, h->value, h->value32);
-  CUDA_TRY(cudaGetLastError());
   k_to_f32<<<grid_stream(h, N), kThreads, 0, h->stream>>>((size_t)N, h->C,
                                                           h->C32);
   CUDA_TRY(cudaGetLastError());
@@ -2478,14 +2475,24 @@ static cgx_status ensure_f32(cgx_handle *h) {
     CUDA_TRY(cudaGetLastError());
   }
   h->off32.filled = h->off32.ok = false;
-  CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
-  k_delta16<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, h->ptr, h->index,
-                                                           h->idx16, h->flag);
-  CUDA_TRY(cudaGetLastError());
-  CUDA_TRY(cudaMemcpyAsync(h->host_scalar, h->flag, sizeof(int),
-                           cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(cudaStreamSynchronize(h->stream));
-  h->compact16 = *(int *)h->host_scalar == 0;
+  // The FP32 CRS copy where neither form holds A: its values, and once per pattern
+  // the 16-bit column offsets.
+  if (!h->band.ok && !h->sa.ok) {
+    k_to_f32<<<grid_stream(h, h->nz), kThreads, 0, h->stream>>>((size_t)h->nz, h->value,
+                                                                h->value32);
+    CUDA_TRY(cudaGetLastError());
+    if (!h->idx16_tried) {
+      CUDA_TRY(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
+      k_delta16<<<grid_stream(h, N), kThreads, 0, h->stream>>>(N, h->ptr, h->index, h->idx16,
+                                                               h->flag);
+      CUDA_TRY(cudaGetLastError());
+      CUDA_TRY(cudaMemcpyAsync(h->host_scalar, h->flag, sizeof(int), cudaMemcpyDeviceToHost,
+                               h->stream));
+      CUDA_TRY(cudaStreamSynchronize(h->stream));
+      h->compact16 = *(int *)h->host_scalar == 0;
+      h->idx16_tried = true;
+    }
+  }
   // The graphs hold pointers and layout choices, not values: a refresh that
   // keeps them keeps the graphs. (Destroying the executable graphs on every
   // refresh cost the first solve after it up to 40 ms of host time now and
@@ -3351,12 +3358,13 @@ cudaError_t gnn_forward(cgx_handle *h, const float *P, bool scaled) {
   const int groups = (N + 15) / 16;
   const int lgrid = std::max(
       1, std::min(h->num_sms * 8, (groups + kLayerWarps - 1) / kLayerWarps));
-  for (int l = 0; l < 3; l++)
-    k_layer<<<lgrid, 32 * kLayerWarps, 0, s>>>(N, h->ptr, h->index, L->ahat, P,
-                                               l, L->h[l], L->h[l + 1],
-                                               keep ? L->agg[l] : nullptr,
-                                               keep ? L->pos[l + 1] : nullptr);
-  k_head<<<grid_for(h, (size_t)N), kThreads, 0, s>>>(N, L->h[3], P, L->o);
+  for (int l = 0; l < 3; l++) {
+    const bool head = l == 2;
+    auto kern = head ? k_layer<true> : k_layer<false>;
+    kern<<<lgrid, 32 * kLayerWarps, 0, s>>>(
+        N, h->ptr, h->index, L->ahat, P, l, L->h[l], head && !keep ? nullptr : L->h[l + 1],
+        keep ? L->agg[l] : nullptr, keep ? L->pos[l + 1] : nullptr, L->o);
+  }
   k_assemble<<<grid_for(h, L->nnzL), kThreads, 0, s>>>(
       L->nnzL, L->grow, L->gcol, L->g2a, L->ahat, L->o, L->ghat, L->dis,
       L->g2t, scaled ? L->gs : nullptr, scaled ? L->gts : nullptr,

@@ -183,4 +183,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar,
   return false;
 }
 
+// The last entry of [j0, j1) whose column is c, or -1. Eight columns are loaded at
+// a time, unconditionally (past the end the last one again).
+__device__ __forceinline__ int last_entry(const int *__restrict__ index, int j0, int j1, int c) {
+  constexpr int U = 8;
+  int at = -1;
+  for (int j = j0; j < j1; j += U) {
+    int col[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) col[u] = __ldg(index + min(j + u, j1 - 1));
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (col[u] == c) at = min(j + u, j1 - 1);
+  }
+  return at;
+}
+
 }  // namespace cgx

@@ -762,10 +762,8 @@ __global__ void __launch_bounds__(kThreads)
                       const double *__restrict__ value, double *C) {
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < N;
        i += gridDim.x * kThreads) {
-    double c = 0.0;
-    for (int j = ptr[i]; j < ptr[i + 1]; j++)
-      if (index[j] == i) c = 1 / value[j];
-    C[i] = c;
+    const int j = last_entry(index, ptr[i], ptr[i + 1], i);
+    C[i] = j >= 0 ? 1 / value[j] : 0.0;
   }
 }
 

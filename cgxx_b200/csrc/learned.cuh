@@ -51,9 +51,8 @@ __global__ void k_inv_sqrt_diag(int N, const int *__restrict__ ptr,
                                 double *dis, int *flag) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
        i += gridDim.x * blockDim.x) {
-    double d = 0.0;
-    for (int j = ptr[i]; j < ptr[i + 1]; j++)
-      if (index[j] == i) d = value[j];
+    const int j = last_entry(index, ptr[i], ptr[i + 1], i);
+    const double d = j >= 0 ? value[j] : 0.0;
     if (!(d > 0.0)) {
       atomicOr(flag, 1);
       dis[i] = 0.0;
@@ -75,17 +74,32 @@ __global__ void k_scaled_rows(int N, const int *__restrict__ ptr,
     const double di = dis[i];
     float s = 0.f, mx = 0.f;
     int deg = 0, lo = 0, up = 0;
-    for (int j = ptr[i]; j < ptr[i + 1]; j++) {
-      const int c = index[j];
-      const float a = (float)(value[j] * di * dis[c]);
-      ahat[j] = a;
-      if (c != i) {
-        s += fabsf(a);
-        mx = fmaxf(mx, fabsf(a));
-        deg++;
+    constexpr int U = 4;
+    const int j1 = ptr[i + 1];
+    for (int j = ptr[i]; j < j1; j += U) {
+      // Unconditional loads, a chunk's columns and values before its scales.
+      int c[U];
+      double v[U], dj[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        c[u] = index[min(j + u, j1 - 1)];
+        v[u] = value[min(j + u, j1 - 1)];
       }
-      lo += c <= i;
-      up += c >= i;
+#pragma unroll
+      for (int u = 0; u < U; u++) dj[u] = dis[c[u]];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (j + u < j1) {
+          const float a = (float)(v[u] * di * dj[u]);
+          ahat[j + u] = a;
+          if (c[u] != i) {
+            s += fabsf(a);
+            mx = fmaxf(mx, fabsf(a));
+            deg++;
+          }
+          lo += c[u] <= i;
+          up += c[u] >= i;
+        }
     }
     feat[i * NIN + 0] = 1.f;
     feat[i * NIN + 1] = s;
@@ -258,21 +272,34 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4],
 // stages X = [h_i ; bf16(agg_i)] (16 x 64, BF16) in shared memory, multiplies
 // by W_l^T on the tensor cores (4 k-steps x 4 n-tiles of m16n8k16, FP32
 // accumulators), adds the bias and writes h_i + relu(pre) as BF16.
+//
+// HEAD (the last layer): also the head outputs o_i = W_h h_i + b_h (FP32), two
+// lanes a node with five outputs each, from the staged rows; h itself is stored
+// only if hout is given (the backward pass reads it). At 96^3 the layer takes 108
+// us with the head, against 89 and 54 for the layer and a pass of its own over h.
 constexpr int kLayerWarps = 8;
-
-__global__ void __launch_bounds__(32 * kLayerWarps)
+// Chunks of four neighbours at 4 CTAs per SM; eight at 3 (2) CTAs: 96^3 86 -> 92
+// (106) us, 2M-point graph 331 -> 375 (407).
+template <bool HEAD>
+__global__ void __launch_bounds__(32 * kLayerWarps, 4)
     k_layer(int N, const int *__restrict__ ptr, const int *__restrict__ index,
             const float *__restrict__ ahat, const float *__restrict__ P,
             int layer, const __nv_bfloat16 *__restrict__ hin,
             __nv_bfloat16 *__restrict__ hout, __nv_bfloat16 *__restrict__ agg_out,
-            uint32_t *__restrict__ mask_out) {
+            uint32_t *__restrict__ mask_out, float *__restrict__ o) {
   __shared__ __align__(16) __nv_bfloat16 sW[W][2 * W + 8];  // W_l[n][k], rows padded (banks)
   __shared__ __align__(16) __nv_bfloat16 sX[kLayerWarps][16][2 * W + 8];  // padded rows
   __shared__ float sB[W];
+  __shared__ __align__(16) float sWh[HEAD ? NOUT : 1][W + 4];  // padded rows (banks)
+  __shared__ float sBh[NOUT];
   const float *Wl = P + OFF_L0 + layer * L_STRIDE;
   for (int t = threadIdx.x; t < W * 2 * W; t += blockDim.x)
     sW[t / (2 * W)][t % (2 * W)] = __float2bfloat16_rn(Wl[t]);
   for (int t = threadIdx.x; t < W; t += blockDim.x) sB[t] = Wl[W * 2 * W + t];
+  if constexpr (HEAD) {
+    for (int t = threadIdx.x; t < NOUT * W; t += blockDim.x) sWh[t / W][t % W] = P[OFF_WH + t];
+    for (int t = threadIdx.x; t < NOUT; t += blockDim.x) sBh[t] = P[OFF_BH + t];
+  }
   __syncthreads();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -300,7 +327,7 @@ __global__ void __launch_bounds__(32 * kLayerWarps)
           float w[4];
           uint4 hv[4];
           int cc[4];
-          // All four entries' columns and weights first, then the four
+          // All of a chunk's columns and weights first, then its
           // gathers: one round trip for each instead of one per entry. The
           // loads are unconditional (past the row's end: its last entry again,
           // weight 0), as a condition would make each a branch.
@@ -390,43 +417,40 @@ __global__ void __launch_bounds__(32 * kLayerWarps)
     for (int q = 0; q < 2; q++) {
       const int task = lane + 32 * q;
       const int r = task >> 2, c4 = task & 3;
-      if (base + r < N)
+      if (base + r < N && (!HEAD || hout))
         reinterpret_cast<uint4 *>(hout)[(size_t)(base + r) * (W / 8) + c4] =
             *reinterpret_cast<const uint4 *>(&sX[warp][r][8 * c4]);
     }
-    __syncwarp();
-  }
-}
-
-// o_i = W_h h_i + b_h (FP32): one thread per node, its 32 features loaded
-// once (four 16-byte loads), W_h from shared memory.
-__global__ void k_head(int N, const __nv_bfloat16 *__restrict__ h,
-                       const float *__restrict__ P, float *__restrict__ o) {
-  __shared__ float sW[NOUT * W + NOUT];
-  for (int t = threadIdx.x; t < NOUT * W + NOUT; t += blockDim.x)
-    sW[t] = P[OFF_WH + t];
-  __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N;
-       i += gridDim.x * blockDim.x) {
-    float hv[W];
-    const uint4 *src = reinterpret_cast<const uint4 *>(h + (size_t)i * W);
+    if constexpr (HEAD) {
+      constexpr int K = NOUT / 2;
+      const int r = lane & 15, k0 = (lane >> 4) * K;
+      float s[K];
 #pragma unroll
-    for (int q = 0; q < W / 8; q++) {
-      const uint4 u = src[q];
-      const __nv_bfloat162 *b2 = reinterpret_cast<const __nv_bfloat162 *>(&u);
+      for (int k = 0; k < K; k++) s[k] = sBh[k0 + k];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        hv[q * 8 + 2 * k] = __low2float(b2[k]);
-        hv[q * 8 + 2 * k + 1] = __high2float(b2[k]);
+      for (int q = 0; q < W / 8; q++) {
+        const uint4 raw = *reinterpret_cast<const uint4 *>(&sX[warp][r][8 * q]);
+        const __nv_bfloat162 *b2 = reinterpret_cast<const __nv_bfloat162 *>(&raw);
+#pragma unroll
+        for (int hf = 0; hf < 2; hf++) {
+          const float h0 = __low2float(b2[2 * hf]), h1 = __high2float(b2[2 * hf]);
+          const float h2 = __low2float(b2[2 * hf + 1]), h3 = __high2float(b2[2 * hf + 1]);
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const float4 w = *reinterpret_cast<const float4 *>(&sWh[k0 + k][8 * q + 4 * hf]);
+            s[k] = fmaf(w.x, h0, s[k]);
+            s[k] = fmaf(w.y, h1, s[k]);
+            s[k] = fmaf(w.z, h2, s[k]);
+            s[k] = fmaf(w.w, h3, s[k]);
+          }
+        }
+      }
+      if (base + r < N) {
+#pragma unroll
+        for (int k = 0; k < K; k++) o[(size_t)(base + r) * NOUT + k0 + k] = s[k];
       }
     }
-#pragma unroll
-    for (int k = 0; k < NOUT; k++) {
-      float s = sW[NOUT * W + k];
-#pragma unroll
-      for (int f = 0; f < W; f++) s = fmaf(sW[k * W + f], hv[f], s);
-      o[(size_t)i * NOUT + k] = s;
-    }
+    __syncwarp();
   }
 }
 
@@ -452,15 +476,20 @@ __global__ void k_assemble(int nnzL, const int *__restrict__ grow,
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnzL;
        e += gridDim.x * blockDim.x) {
     const int i = grow[e], j = gcol[e];
+    // Rows of o are 8-byte aligned: pairs, all loaded before the first use.
+    const float2 *oi = reinterpret_cast<const float2 *>(o + (size_t)i * NOUT);
+    const float2 *oj = reinterpret_cast<const float2 *>(o + (size_t)j * NOUT + 2 + RANK);
+    const float2 a = oi[0], u0 = oi[1], u1 = oi[2], v0 = oj[0], v1 = oj[1];
+    const float w = fabsf(ahat[g2a[e]]);
     float v;
     if (i == j) {
-      v = softplus(o[i * NOUT + 1] + DIAG_OFFSET);
+      v = softplus(a.y + DIAG_OFFSET);
     } else {
-      float uv = 0.f;
-#pragma unroll
-      for (int k = 0; k < RANK; k++)
-        uv = fmaf(o[i * NOUT + 2 + k], o[j * NOUT + 2 + RANK + k], uv);
-      v = fabsf(ahat[g2a[e]]) * (o[i * NOUT + 0] + uv);
+      float uv = fmaf(u0.x, v0.x, 0.f);
+      uv = fmaf(u0.y, v0.y, uv);
+      uv = fmaf(u1.x, v1.x, uv);
+      uv = fmaf(u1.y, v1.y, uv);
+      v = w * (a.x + uv);
     }
     ghat[e] = v;
     if (gbv) {  // the band copy of G (BF16), which serves G and G^T
