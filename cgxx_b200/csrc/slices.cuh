@@ -11,9 +11,10 @@
 // row's products are added in that order; rows shorter than their slice end in
 // entries of column -1, which are skipped. A geometric graph of mean degree 12
 // (rows of 1-34 entries) pads by 6 % in A and 19 and 25 % in G and G^T in windows
-// of 1024 rows (unsorted 52, 94 and 94 %; by length alone 3, 41 and 46 %). Every
-// second step's slices run from the shortest to the longest, which evens out the
-// warps of a CTA.
+// of 1024 rows (unsorted 52, 94 and 94 %; by length alone 3, 41 and 46 %). So
+// that the warps of a CTA get the same work over its steps, every second step's
+// slices run from the shortest to the longest, and each pair of steps starts with
+// other warps (the pairs' starts spread over them).
 //
 // Against the tiles of k_crs (values and indices through shared memory): every
 // load of the matrix is one run of 64 to 256 bytes per warp, straight to
@@ -23,15 +24,15 @@
 // then DRAM. us per iteration of the persistent solves on graphs, graph of kernels
 // -> sorted slices (1,000,003 points: 149 MB in FP64, 23 us at the measured 6.54
 // TB/s; 2,000,000 points learned: 400 MB, 61 us):
-//   FP64     5,003: 19.6 -> 8.1   400,009: 37 -> 22   1,000,003: 71 -> 43   2M: 122 -> 82
-//   mixed    5,003: 21.9 -> 8.6   400,009: 31 -> 19   2M: 85 -> 55
-//   learned  5,003: 28.8 -> 15    400,009: 55 -> 40   2M: 161 -> 121
+//   FP64     5,003: 19.6 -> 8.1   300,007: - -> 17   1,000,003: 71 -> 40   2M: 122 -> 80
+//   mixed    5,003: 21.9 -> 8.6   300,007: - -> 15   1,000,003: - -> 31   2M: 85 -> 54
+//   learned  5,003: 28.8 -> 15    300,007: - -> 31   1,000,003: - -> 65   2M: 161 -> 112
 // Steps on the way (FP64 at 1M / learned at 2M): matrix through L1, 192 KB of
 // resident vectors 52 / -; kept out of L1, 128-160 KB 47 / 144; loads past a
 // slice's width predicated off instead of repeated 41.5 / 139; a chunk ahead 43 /
-// 121 (4 entries at a time: 44 / 142; FP64 with 8: spills, 78). Tried without gain:
-// an L2 evict-last policy on part of the matrix, L2 prefetch of the next slice or
-// of the next product's first steps, 512-thread CTAs.
+// 121; the pairs' starts spread 40 / 112. (4 entries at a time 44 / 142; FP64 with 8
+// spills, 78.) Tried without gain: an L2 evict-last policy on part of the matrix, L2
+// prefetch of the next slice or of the next product's first steps, 512-thread CTAs.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -93,8 +94,11 @@ __global__ void __launch_bounds__(kSliceWindow)
     }
   __syncthreads();
   mine = key[t];
-  const bool full = w0 + T <= N, turn = full && ((blockIdx.x / grid) & 1);
-  const int slot = turn ? w0 + (T - 32 - (t & ~31)) + (t & 31) : i;
+  // Where the window's slices go (see above); the last, partial window's stay.
+  const int S = T / 32, steps = ((int)gridDim.x + grid - 1) / grid, step = blockIdx.x / grid;
+  const int rank = (step & 1) ? S - 1 - (t >> 5) : t >> 5;
+  const int shift = (step >> 1) * S / ((steps + 1) >> 1);
+  const int slot = w0 + T <= N ? w0 + (rank + shift) % S * 32 + (t & 31) : i;
   int len = 0;
   if (i < N) {
     const int row = w0 + T - 1 - (int)(mine & 4095u);
