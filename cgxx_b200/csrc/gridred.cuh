@@ -19,8 +19,8 @@
 // eight copies), and one CTA that collects the slots and answers into a
 // mailbox per CTA (3.1-4.0 us).
 //
-// Every wait is bounded (kSyncPolls polls); a CTA that gives up reports false
-// and its kernel leaves the loop, sets kErrGridSync and returns.
+// Every wait on a grid is bounded (kSyncPolls polls); a CTA that gives up reports
+// false and its kernel leaves the loop, sets kErrGridSync and returns.
 #pragma once
 
 #include "device.cuh"
@@ -156,10 +156,13 @@ __device__ __forceinline__ bool grid_sum(RedMem *m, unsigned &round,
 
 // The same for a launch that is one thread-block cluster (at most kClusterCtas
 // CTAs): the partials go straight into every CTA's shared memory, and the
-// cluster's hardware barrier, which needs no polls, makes them visible. It always
-// ends, as the CTAs of a cluster run together and take the same decisions. Before
-// a CTA returns, cluster_sync (another CTA may still write to it). A fused
-// iteration on 64^2 rows, two sums, takes 3.0 us with it and 4.8 on the grid.
+// cluster's hardware barrier, which needs no polls, makes them visible. It has no
+// limit, but always ends, as the CTAs of a cluster run together and take the same
+// decisions. A CTA's shared memory may be written only while it runs: every
+// kernel calls cluster_sync before its first cluster_sum (the CTAs are scheduled
+// together, but one without rows would store before a later one has started) and
+// before a CTA returns (another may still write to it). A fused iteration on 64^2
+// rows, two sums, takes 3.0 us with it and 4.8 on the grid.
 constexpr int kClusterCtas = 16;
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");

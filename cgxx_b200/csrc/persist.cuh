@@ -49,9 +49,11 @@
 // to 17.7 (128^3), 45.0 to 38.1 (160^3), and learned 18.2 to 16.4, 41.0 to 32.5
 // and 71.5 to 70.3; 24^3: 7.5 to 4.8 and 9.3 to 6.6.
 //
-// Every wait is bounded: a CTA that gives up sets kErrGridSync in
-// CgState::error and leaves the loop, so the launch always ends and the host
-// reports CGX_ERROR_DEVICE.
+// Every wait of a cooperative launch is bounded: a CTA that gives up sets
+// kErrGridSync in CgState::error and leaves the loop, so the launch always ends
+// and the host reports CGX_ERROR_DEVICE. A cluster launch waits at the hardware's
+// cluster barrier, which has no limit: all of its CTAs run together and take the
+// same decisions from the same sums, so each of them reaches every barrier.
 #pragma once
 
 #include "band.cuh"
@@ -553,7 +555,10 @@ __global__ void __launch_bounds__(TPB, 1)
     bring(sr, a.nr, a.r);
     bring(sd, a.nd, a.d);
     bring(scd, a.nc, a.C);
-    __syncthreads();
+    if (CLUSTER)
+      cluster_sync();  // cluster_sum needs all of its CTAs started
+    else
+      __syncthreads();
   }
   // C is written in this launch only with kPerm (then not the read-only path).
   auto cval = [&](int k, int o, int i) {
@@ -711,6 +716,7 @@ __global__ void __launch_bounds__(TPB, 1)
     for (; i + TPB < hi; k += 2, i += 2 * TPB) f(IntTag<2>{}, k, i);
     if (i < hi) f(IntTag<1>{}, k, i);
   };
+  if (CLUSTER) cluster_sync();  // cluster_sum needs all of its CTAs started
   // The start's p = z: the first iteration forms p = z and leaves d at 0.
   const float *po = a.p, *ro = a.r;
   float *pn = a.p2, *rn = a.r2;

@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(TPB, 1) k_solve64(Mat A, Solve64Args a, CgStat
       if (k < a.nc) scd[k * TPB + threadIdx.x] = a.C ? a.C[i] : 1.0;
     }
   }
-  if (PERM) ok = sync_over<CLUSTER, TPB>(a.red, round);  // p is read across CTAs
+  // p is read across CTAs; a cluster's sums need all of its CTAs started.
+  if (PERM || CLUSTER) ok = sync_over<CLUSTER, TPB>(a.red, round);
   // C of step k: shared, global, or 1 (1 * r is r, exactly).
   auto c_at = [&](int k, int i) {
     return k < a.nc ? scd[k * TPB + threadIdx.x] : a.C ? __ldca(a.C + i) : 1.0;
