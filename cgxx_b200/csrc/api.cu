@@ -558,6 +558,15 @@ __global__ void k_loop_guard(CgState *st) {
 // ---------------------------------------------------------------------------
 // Launch helpers
 
+// The dynamic shared memory that a kernel may be launched with. The limit belongs
+// to the kernel on its device, not to a handle: every caller sets the same number,
+// whatever its own launch takes, as another thread's smaller one between this
+// call and the launch would make the launch fail.
+constexpr size_t kSmemLimit = 200 << 10;
+static cudaError_t raise_smem_limit(const void *kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+}
+
 // Staged CRS SpMV over any CRS view (A itself, or the learned factor's G and
 // G^T, whose rows are subsets of A's rows so A's tile capacity bounds them).
 template <typename VT, typename IT, typename Op>
@@ -567,10 +576,7 @@ static cudaError_t launch_crs_view(cgx_handle *h, CrsView<VT, IT> A,
     const size_t smem = 16 * kWarps + kWarps * crs_stage_bytes<VT, IT>(A.warp_cap);
     auto kern = k_crs_warp<VT, IT, Op>;
     cudaError_t e;
-    if (smem > 48 * 1024 &&
-        (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
-      return e;
+    if (smem > 48 * 1024 && (e = raise_smem_limit((const void *)kern)) != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
     if (e != cudaSuccess) return e;
@@ -584,8 +590,7 @@ static cudaError_t launch_crs_view(cgx_handle *h, CrsView<VT, IT> A,
   const size_t smem = crs_smem_bytes<VT, IT>(cap);
   auto kern = k_crs<VT, IT, Op>;
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(
-        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = raise_smem_limit((const void *)kern);
     if (e != cudaSuccess) return e;
   }
   int per_sm = 0;
@@ -620,9 +625,7 @@ static cudaError_t launch_spmv(cgx_handle *h, const double *x, Op op) {
       const size_t smem = ell_smem_bytes<double>(h->ell_width);
       auto kern = k_ell_tma<double, Op>;
       cudaError_t e;
-      if (smem > 48 * 1024 &&
-          (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem)) != cudaSuccess)
+      if (smem > 48 * 1024 && (e = raise_smem_limit((const void *)kern)) != cudaSuccess)
         return e;
       int per_sm = 0;
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
@@ -1918,8 +1921,7 @@ static cgx_status ensure_band64(cgx_handle *h, const Rows &A, int loop, bool *us
 // of resident vectors.
 static cudaError_t launch_coop(cgx_handle *h, const void *kern, int grid, int T, size_t smem,
                                void **args) {
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = raise_smem_limit(kern);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->red, 0, kRedZeroBytes, h->stream);
   if (e != cudaSuccess) return e;
   return cudaLaunchCooperativeKernel(kern, grid, T, args, smem, h->stream);
@@ -1943,7 +1945,7 @@ static cudaError_t launch_resident(cgx_handle *h, void (*kern)(Args...), int gri
   *ran = false;
   cudaError_t e;
   if (CLUSTER) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = raise_smem_limit((const void *)kern);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg{};
@@ -1983,6 +1985,9 @@ constexpr int kSolve64Resident = 192 << 10;
 
 // The same on sorted slices, whose gathers need more of the L1 (slices.cuh).
 constexpr int kSliceResident = 160 << 10;
+static_assert(kSolve64Resident <= kSmemLimit && kSliceResident <= kSmemLimit &&
+                  kInnerResident <= kSmemLimit,
+              "resident vectors");
 
 // The loop of a plain FP64 solve as one cooperative launch, after the set-up
 // kernel. *ran = false when the GPU cannot hold the grid at once (a device
