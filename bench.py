@@ -362,12 +362,10 @@ def persist_roofline(args, results, N, peak, peak_kind):
     return out
 
 
-def plain_persistent(args, N):
-    """Whether the plain solve's loop is one persistent launch: the default
-    loop's on every workload here, but for the 7-point grids of 0.7M to 1.1M rows
-    (kSolve64FusedMaxRows, kSolve64SplitMinRows)."""
-    return args.loop in ("graph", "persistent", "split") and (bool(args.graph) or not (
-        args.loop == "graph" and args.stencil == 7 and 700000 < N < 1100000))
+def plain_persistent(args):
+    """Whether the plain solve's loop is one persistent launch, as in these loop
+    modes on every workload here."""
+    return args.loop in ("graph", "persistent", "split")
 
 
 def peaks():
@@ -637,7 +635,7 @@ def our_arm(args, world, rank, local):
     # refinement check (outer + 1), and per refinement step its start, the
     # inner solve and the update of x; the learned path adds its set-up
     # (2 kernels), inference (5) and the start's apply (2 per step).
-    if args.path == "plain" and plain_persistent(args, N):
+    if args.path == "plain" and plain_persistent(args):
         per_solve = 3                               # fill, set-up, one launch
     elif args.path == "plain":
         per_solve = 2 + 4 * iters                   # fill, set-up, 3 fused + guard

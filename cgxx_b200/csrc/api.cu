@@ -1844,19 +1844,16 @@ static cgx_status band64_alloc(cgx_handle *h, int KP, bool *got) {
 //     128^3                  153     - | 116        110 | 124
 //   27-point, symmetric half stored:
 //     96^3                   73.4    - | 39.9       35.6 | 33.2
-// So: fused up to 0.7M rows with few offsets (0.2M with many), 256-thread CTAs
+// Fused | split where they cross, Jacobi, against kernels one by one: 7-point 90^3
+// 13.5 | 15.3 (26.8), 96^3 14.9 | 16.8 (35.1), 104^3 18.1 | 19.7 (42.4), 108^3 22.2 |
+// 21.2 (46.4), 112^3 29.3 | 22.6 (50.2); 5-point 1000^2 15.1 | 16.6 (30.9), 1100^2
+// 17.3 | 17.9 (39.1), 1200^2 23.5 | 20.6 (44.7).
+// So: fused up to 1.2M rows with few offsets (0.2M with many), 256-thread CTAs
 // up to one pass of them; split beyond, 512 threads where the offsets are all
 // stored and many (their loads need the registers).
-constexpr int kSolve64FusedMaxRows = 700000;
+constexpr int kSolve64FusedMaxRows = 1200000;
 constexpr int kSolve64FusedMaxRowsWide = 200000;
 constexpr int kSolve64NarrowCtaRows = 148 * 256;
-// Few offsets, between kSolve64FusedMaxRows and this: the graph of kernels. The
-// fused form would be faster here too (96^3: 15.2 us per iteration against 36),
-// but the project's bar for the learned solve is twice the plain solve's speed
-// on 96^3 fields (test_learned_twice_as_fast_as_plain_on_heldout_fields), and
-// the learned solve (4.1 ms a field) meets it against the graph (2.9x), not
-// against this form (1.3x).
-constexpr int kSolve64SplitMinRows = 1100000;
 // The smallest systems run as one cluster of up to 16 CTAs, whose barriers cost
 // less than half of the grid's (us per iteration, cooperative grid -> cluster with
 // 256 | 512 threads: 5-point 32^2 4.9 -> 2.8 | 3.2, 64^2 4.8 -> 3.0 | 3.1, 90^2 4.8
@@ -1870,17 +1867,12 @@ constexpr int kClusterMaxRows = 16384, kClusterMaxRowsWide = 8192;
 // of them on (160^3, 131 MB: 78.3 -> 76.3 us; 128^3, 67 MB: 37.7 -> 36.4;
 // 112^3, 45 MB, which stay in L2: 23.1 -> 24.2).
 constexpr size_t kSolve64PrefetchBytes = (size_t)60 << 20;
-// At most the seven offsets of the 7-point stencil.
-static bool few_offsets(const cgx_handle *h) {
-  return h->b64.planned && !h->b64.all.empty() && (int)h->b64.all.size() <= 7;
-}
 
-// The by-offset values of the current matrix, for a solve in the given loop
-// mode. They are used when they take no more bytes than the entries of the
-// uploaded layout (12 each): a matrix whose offsets are mostly empty stays on
-// its rows.
+// The by-offset values of the current matrix. They are used when they take no more
+// bytes than the entries of the uploaded layout (12 each): a matrix whose offsets
+// are mostly empty stays on its rows.
 template <typename Rows>
-static cgx_status ensure_band64(cgx_handle *h, const Rows &A, int loop, bool *use) {
+static cgx_status ensure_band64(cgx_handle *h, const Rows &A, bool *use) {
   Band64 &B = h->b64;
   *use = false;
   if (!B.planned) {
@@ -1888,9 +1880,6 @@ static cgx_status ensure_band64(cgx_handle *h, const Rows &A, int loop, bool *us
     B.half = half_offsets(B.all);
     B.planned = true;
   }
-  if (loop == CGX_LOOP_GRAPH && few_offsets(h) && h->N > kSolve64FusedMaxRows &&
-      h->N < kSolve64SplitMinRows)
-    return CGX_SUCCESS;
   *use = B.ok;
   if (B.filled) return CGX_SUCCESS;
   B.ok = false;
@@ -2217,9 +2206,8 @@ template <typename Rows>
 static cgx_status solve_persistent64(cgx_handle *h, const Rows &A, const cgx_options &o,
                                      bool jacobi, bool *ran) {
   bool band = false, slices = false;
-  CGX_TRY(ensure_band64(h, A, o.loop, &band));
-  // A matrix of few offsets that its own rule leaves to the graph stays there.
-  if (!band && !h->b64.ok && !few_offsets(h)) CGX_TRY(ensure_slices(h, A, &slices));
+  CGX_TRY(ensure_band64(h, A, &band));
+  if (!band) CGX_TRY(ensure_slices(h, A, &slices));
   if (!band && !slices) return CGX_SUCCESS;
   reset_host_state(h, o.max_iterations, o.tolerance, false, 0);
   CGX_TRY(push_state(h));

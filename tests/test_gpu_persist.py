@@ -212,3 +212,29 @@ def test_plain_forms_stop_as_the_kernels_do(handle, loop):
     handle.fill_vector("X", 0.0)
     r = handle.solve(max_iterations=7, tolerance=1e-11, loop=loop)
     assert r["iterations"] == 7 and r["converged"] == 0
+
+
+@pytest.mark.parametrize("kind,N", [("half4", 729001), ("all7", 1048577), ("half3", 1199999),
+                                    ("half4", 1200001), ("reversed", 884736)])
+def test_plain_default_takes_a_persistent_form(handle, kind, N):
+    """0.7M to 1.2M rows and at most seven offsets: ten iterations of the default
+    loop agree with the chunked kernels (the bound of
+    test_plain_forms_agree_with_the_kernels) and take less time; the default loop
+    run as those kernels takes as long as they do."""
+    A = fp64_matrix(kind, N)
+    b, _ = G.rhs_for(A, seed=3)
+    upload(handle, A, "coo" if kind == "reversed" else ("crs", "ell")[N % 2])
+    handle.jacobi_from_matrix()
+    handle.set_vector("K", b)
+    x, ms = {}, {}
+    for loop in (cg.LOOP_CHUNKED, cg.LOOP_GRAPH):
+        for _ in range(4):  # the first includes the layout
+            handle.fill_vector("X", 0.25)
+            r = handle.solve(max_iterations=10, tolerance=1e-30, loop=loop)
+            assert r["iterations"] == 10
+            ms[loop] = min(ms.get(loop, 1e9), r["solve_ms"])
+        x[loop] = handle.get_vector("X")
+    want = x[cg.LOOP_CHUNKED]
+    assert np.linalg.norm(x[cg.LOOP_GRAPH] - want) <= \
+        20 * KAPPA * N * 2.0 ** -53 * np.linalg.norm(want)
+    assert ms[cg.LOOP_GRAPH] < 0.8 * ms[cg.LOOP_CHUNKED], ms
