@@ -22,6 +22,8 @@
 // -> 157.
 #pragma once
 
+#include <cfloat>
+
 #include "learned.cuh"
 
 namespace cgx {
@@ -265,12 +267,18 @@ __device__ __forceinline__ float4 masked(float4 v, uint32_t m) {
 }
 
 // v as a sum of three BF16 values, largest first (24 bits: exact but for values
-// whose last bits fall below the smallest FP32 numbers).
+// whose last bits fall below the smallest FP32 numbers). Above BF16's largest number
+// the first term is rounded towards zero; an infinite v is its first term alone, as
+// the difference would be NaN.
 __device__ __forceinline__ void split3(float v, __nv_bfloat16 (&s)[3]) {
   s[0] = __float2bfloat16_rn(v);
-  v -= __bfloat162float(s[0]);
-  s[1] = __float2bfloat16_rn(v);
-  s[2] = __float2bfloat16_rn(v - __bfloat162float(s[1]));
+  float rest = v - __bfloat162float(s[0]);
+  if (fabsf(__bfloat162float(s[0])) > 3.4e38f) {  // infinite
+    s[0] = __float2bfloat16_rz(v);
+    rest = fabsf(v) > FLT_MAX ? 0.f : v - __bfloat162float(s[0]);
+  }
+  s[1] = __float2bfloat16_rn(rest);
+  s[2] = __float2bfloat16_rn(rest - __bfloat162float(s[1]));
 }
 
 // Four 8 x 8 matrices of 16-bit elements from shared memory, lane l giving the
