@@ -397,20 +397,28 @@ static void dev_free(cgx_handle *h, void *p) {
   h->spare.emplace(it->second, p);
 }
 
+// The same, back to the device at once.
+static void dev_release(cgx_handle *h, void *p) {
+  if (!p) return;
+  h->block_size.erase(p);
+  cudaFree(p);
+}
+
 template <typename VT>
-static void slices_free(cgx_handle *h, SliceArrays<VT> &S) {
-  dev_free(h, S.plan);
-  dev_free(h, S.mem);
+static void slices_free(cgx_handle *h, SliceArrays<VT> &S,
+                        void (*give)(cgx_handle *, void *) = dev_free) {
+  give(h, S.plan);
+  give(h, S.mem);
   S = SliceArrays<VT>{};
 }
 
-static void slices_free(cgx_handle *h, Slices &S) {
-  slices_free(h, S.a64);
-  slices_free(h, S.a32);
-  slices_free(h, S.g);
-  slices_free(h, S.gt);
-  dev_free(h, S.mem);
-  dev_free(h, S.vec_mem);
+static void slices_free(cgx_handle *h, Slices &S, void (*give)(cgx_handle *, void *) = dev_free) {
+  slices_free(h, S.a64, give);
+  slices_free(h, S.a32, give);
+  slices_free(h, S.g, give);
+  slices_free(h, S.gt, give);
+  give(h, S.mem);
+  give(h, S.vec_mem);
   S = Slices{};
 }
 
@@ -2157,12 +2165,22 @@ static cgx_status slices_matrix(cgx_handle *h, const Rows &A, size_t nnz, double
 // Padding that the slices of A, and of the factor, may add.
 constexpr double kSlicesMost = 1.25, kSlicesMostFactor = 2.0;
 
+// Without slices of A the slot order serves nothing: its memory (48 bytes a row and
+// the plans) goes back to the device, and the matrix stays without.
+static void slices_give_up(cgx_handle *h) {
+  Slices &S = h->sl;
+  if (S.a64.ok || S.a32.ok) return;
+  slices_free(h, S, dev_release);
+  S.planned = true;
+}
+
 // FP64 slices of the current matrix; *use = false if it does not fit them.
 template <typename Rows>
 static cgx_status ensure_slices(cgx_handle *h, const Rows &A, bool *use) {
   CGX_TRY(ensure_slots(h, A));
   if (h->sl.ok) CGX_TRY(slices_matrix(h, A, (size_t)h->nz, kSlicesMost, h->sl.a64));
   *use = h->sl.a64.ok;
+  slices_give_up(h);
   return CGX_SUCCESS;
 }
 
@@ -2810,13 +2828,18 @@ static cgx_status ensure_inner_slices(cgx_handle *h, bool want_learned, bool *us
     return CGX_SUCCESS;
   const RowsCrs A{h->ptr, h->index, h->value};
   CGX_TRY(ensure_slots(h, A));
-  if (!S.ok) return CGX_SUCCESS;
-  CGX_TRY(slices_matrix(h, A, (size_t)h->nz, kSlicesMost, S.a32));
+  if (S.ok) CGX_TRY(slices_matrix(h, A, (size_t)h->nz, kSlicesMost, S.a32));
+  slices_give_up(h);
   if (want_learned && S.a32.ok) {
     const learned::RowsFactor<false> G{L->gptr, L->gcol, nullptr, L->ghat, L->dis};
     const learned::RowsFactor<true> GT{L->tptr, L->tcol, L->t2g, L->ghat, L->dis};
     CGX_TRY(slices_matrix(h, G, (size_t)L->nnzL, kSlicesMostFactor, S.g));
-    CGX_TRY(slices_matrix(h, GT, (size_t)L->nnzL, kSlicesMostFactor, S.gt));
+    if (S.g.ok) CGX_TRY(slices_matrix(h, GT, (size_t)L->nnzL, kSlicesMostFactor, S.gt));
+    if (!S.g.ok || !S.gt.ok) {  // one alone serves nothing
+      slices_free(h, S.g, dev_release);
+      slices_free(h, S.gt, dev_release);
+      S.g.planned = S.gt.planned = true;
+    }
   }
   *use = S.a32.ok && (!want_learned || (S.g.ok && S.gt.ok));
   return CGX_SUCCESS;

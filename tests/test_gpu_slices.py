@@ -134,3 +134,30 @@ def test_inner_solves_match_the_kernels(name, make, learned):
                 its[loop] = r["iterations"]
             assert abs(its[cg.LOOP_GRAPH] - its[cg.LOOP_KERNELS]) <= 0.02 * its[cg.LOOP_KERNELS] + 2
         net.close()
+
+
+def test_rejected_slices_keep_no_memory():
+    """Eight rows of 200 entries among every 1024 of one: the slices would more than
+    double the entries, so the solve stays on the rows and what was laid out on the
+    way (48 bytes a row) is given back. Kernels and graphs are loaded by a small
+    solve first; they and the flags may take a tenth of those bytes."""
+    import torch
+
+    def solve(N):
+        rows = np.arange(0, N, 128)
+        r = np.concatenate([np.arange(N), np.repeat(rows, 199)])
+        c = np.concatenate([np.arange(N), (rows[:, None] + 31 * np.arange(1, 200)).ravel() % N])
+        A = G.crs_from_unsorted(N, r, c, np.where(r == c, 4.0, 1e-3))
+        h = cg.Handle(0)
+        h.upload_crs(A.ptr, A.index, A.value)
+        h.fill_vector("K", 1.0)
+        h.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        h.solve(max_iterations=5, tolerance=1e-30, preconditioner=cg.PRECOND_NONE)
+        taken = free - torch.cuda.mem_get_info()[0]
+        h.close()
+        return taken
+
+    solve(20000)
+    N = 2000000
+    assert solve(N) <= 48 * N / 10
