@@ -279,9 +279,13 @@ struct cgx_handle {
   // Values by offset of the persistent plain solves.
   Band64 b64;
   Slices sl;
+  int *offset_table = nullptr;
+  unsigned long long *counts = nullptr;
+  bool keep_layouts = false;  // a solve is using off32, b64 or sl (KeepLayouts)
   RedMem *red = nullptr;  // barrier state of the persistent solves (gridred.cuh)
 
-  // Scratch: state, partial sums, dot result, validation flag, barrier state.
+  // Scratch: state, partial sums, dot result, validation flag, barrier state, and
+  // what the layouts' set-up fills (k_band_offsets, the symmetry checks).
   void *scratch = nullptr;
   CgState *st = nullptr;
   double *partials = nullptr;
@@ -367,37 +371,7 @@ static void release_spare(cgx_handle *h) {
   h->spare.clear();
 }
 
-static cudaError_t dev_alloc(cgx_handle *h, void **p, size_t bytes) {
-  *p = nullptr;
-  if (bytes == 0) bytes = 1;
-  auto it = h->spare.lower_bound(bytes);
-  if (it != h->spare.end() && it->first <= bytes + bytes / 4 + (1u << 20)) {
-    *p = it->second;
-    h->spare.erase(it);
-    return cudaSuccess;
-  }
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && !h->spare.empty()) {
-    cudaGetLastError();
-    release_spare(h);
-    e = cudaMalloc(p, bytes);
-  }
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return e;
-  }
-  h->block_size[*p] = bytes;
-  return cudaSuccess;
-}
-
-static void dev_free(cgx_handle *h, void *p) {
-  if (!p) return;
-  auto it = h->block_size.find(p);
-  if (it == h->block_size.end()) return;
-  h->spare.emplace(it->second, p);
-}
-
-// The same, back to the device at once.
+// A block back to the device at once.
 static void dev_release(cgx_handle *h, void *p) {
   if (!p) return;
   h->block_size.erase(p);
@@ -420,6 +394,61 @@ static void slices_free(cgx_handle *h, Slices &S, void (*give)(cgx_handle *, voi
   give(h, S.mem);
   give(h, S.vec_mem);
   S = Slices{};
+}
+
+// The copies that only make solves faster (values by offset, sorted slices), given
+// back when an allocation that a call cannot do without finds no room. The next
+// solve lays them out again if there is. False if there were none, or a solve is
+// using them (KeepLayouts).
+static bool release_layouts(cgx_handle *h) {
+  if (h->keep_layouts || (!h->b64.mem && !h->off32.U && !h->sl.mem && !h->sl.vec_mem)) return false;
+  dev_release(h, h->b64.mem);
+  h->b64 = Band64{};
+  dev_release(h, h->off32.U);
+  h->off32 = Off32{};
+  slices_free(h, h->sl, dev_release);
+  return true;
+}
+
+struct KeepLayouts {
+  cgx_handle *h;
+  const bool was;
+  explicit KeepLayouts(cgx_handle *hd) : h(hd), was(hd->keep_layouts) { h->keep_layouts = true; }
+  ~KeepLayouts() { h->keep_layouts = was; }
+};
+
+static cudaError_t dev_alloc(cgx_handle *h, void **p, size_t bytes) {
+  *p = nullptr;
+  if (bytes == 0) bytes = 1;
+  auto it = h->spare.lower_bound(bytes);
+  if (it != h->spare.end() && it->first <= bytes + bytes / 4 + (1u << 20)) {
+    *p = it->second;
+    h->spare.erase(it);
+    return cudaSuccess;
+  }
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && !h->spare.empty()) {
+    cudaGetLastError();
+    release_spare(h);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaErrorMemoryAllocation && release_layouts(h)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    return e;
+  }
+  h->block_size[*p] = bytes;
+  return cudaSuccess;
+}
+
+static void dev_free(cgx_handle *h, void *p) {
+  if (!p) return;
+  auto it = h->block_size.find(p);
+  if (it == h->block_size.end()) return;
+  h->spare.emplace(it->second, p);
 }
 
 static void drop_graphs(cgx_handle *h) {
@@ -1002,6 +1031,8 @@ cgx_status cgx_create(cgx_handle **out, int device) {
   size_t o_dot = c.take<double>(4);
   size_t o_flag = c.take<int>(4);
   size_t o_red = c.take<RedMem>(1);
+  size_t o_tab = c.take<int>(kBandTable);
+  size_t o_cnt = c.take<unsigned long long>(2);
   if ((e = cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking)) !=
           cudaSuccess ||
       (e = cudaMalloc(&h->scratch, c.off)) != cudaSuccess ||
@@ -1023,6 +1054,8 @@ cgx_status cgx_create(cgx_handle **out, int device) {
   h->dot_out = (double *)(base + o_dot);
   h->flag = (int *)(base + o_flag);
   h->red = (RedMem *)(base + o_red);
+  h->offset_table = (int *)(base + o_tab);
+  h->counts = (unsigned long long *)(base + o_cnt);
   e = cudaMemsetAsync(h->scratch, 0, c.off, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
@@ -1719,8 +1752,7 @@ template <typename Rows>
 static cgx_status band_offsets(cgx_handle *h, const Rows &A, std::vector<int> &D) {
   D.clear();
   const int N = h->N;
-  int *table = nullptr;
-  CUDA_TRY(dev_alloc(h, (void **)&table, sizeof(int) * kBandTable));
+  int *table = h->offset_table;
   std::vector<int> host(kBandTable, kBandEmpty);
   int flag = 0;
   cudaError_t e = cudaMemcpyAsync(table, host.data(), sizeof(int) * kBandTable,
@@ -1737,7 +1769,6 @@ static cgx_status band_offsets(cgx_handle *h, const Rows &A, std::vector<int> &D
     e = cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost,
                         h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  dev_free(h, table);
   CUDA_TRY(e);
   if (flag) return CGX_SUCCESS;
   for (int v : host)
@@ -1780,8 +1811,7 @@ static cgx_status band64_fill(cgx_handle *h, const Rows &A, const std::vector<in
   Band64Offsets o{};
   o.K = (int)D.size();
   for (int k = 0; k < o.K; k++) o.d[k] = D[k];
-  unsigned long long *counts = nullptr;
-  CUDA_TRY(dev_alloc(h, (void **)&counts, 2 * sizeof(unsigned long long)));
+  unsigned long long *counts = h->counts;
   unsigned long long hc[2] = {0, 0};
   int flag = 0;
   cudaError_t e = cudaMemsetAsync(U, 0, sizeof(VT) * KP * ld, h->stream);
@@ -1801,7 +1831,6 @@ static cgx_status band64_fill(cgx_handle *h, const Rows &A, const std::vector<in
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  dev_free(h, counts);
   CUDA_TRY(e);
   *fits = flag == 0 && (!SYM || hc[0] == hc[1]);
   return CGX_SUCCESS;
@@ -2240,6 +2269,7 @@ static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
   if (jacobi && !h->c_valid)
     return fail(CGX_ERROR_INVALID_STATE, "Jacobi preconditioner not set");
   cudaStream_t s = h->stream;
+  KeepLayouts keep(h);
   // One persistent launch on the by-offset values; PERSISTENT and PERSISTENT_SPLIT
   // force its fused or split form, and run as GRAPH on other matrices.
   const bool want_persist = o.loop == CGX_LOOP_GRAPH || o.loop == CGX_LOOP_PERSISTENT ||
@@ -2353,8 +2383,7 @@ static cgx_status band_fill(cgx_handle *h, Band &B) {
   B.ok = false;
   const size_t bytes = sizeof(float) * (size_t)N * kBandMaxK;
   if (!B.U) CUDA_TRY(dev_alloc(h, (void **)&B.U, bytes));
-  unsigned long long *counts = nullptr;
-  CUDA_TRY(dev_alloc(h, (void **)&counts, 2 * sizeof(unsigned long long)));
+  unsigned long long *counts = h->counts;
   BandOffsets o{};
   o.K = B.K;
   for (int k = 0; k < B.K; k++) o.d[k] = B.d[k];
@@ -2380,7 +2409,6 @@ static cgx_status band_fill(cgx_handle *h, Band &B) {
     e = cudaMemcpyAsync(&flag, h->flag, sizeof(int), cudaMemcpyDeviceToHost,
                         h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  dev_free(h, counts);
   CUDA_TRY(e);
   B.ok = flag == 0 && hc[0] == hc[1];
   return CGX_SUCCESS;
@@ -2909,6 +2937,7 @@ static cgx_status solve_mixed(cgx_handle *h, const cgx_options &o,
   cudaStream_t s = h->stream;
   CUDA_TRY(cudaEventRecord(h->ev[6], s));
   CGX_TRY(ensure_f32(h));
+  KeepLayouts keep(h);
 
   // The persistent inner solves (persist.cuh); the fused form's start also
   // stores z.
