@@ -2248,7 +2248,8 @@ static cudaError_t launch_slices64(cgx_handle *h, bool jacobi, bool *ran) {
 }
 
 // The persistent plain solve of the matrix given by its rows, if it has a form
-// for it.
+// for it. ev[0] is recorded behind the layout, which a solve on new values lays out
+// once: solve_ms is the solve, as in the other loops.
 template <typename Rows>
 static cgx_status solve_persistent64(cgx_handle *h, const Rows &A, const cgx_options &o,
                                      bool jacobi, bool *ran) {
@@ -2258,6 +2259,7 @@ static cgx_status solve_persistent64(cgx_handle *h, const Rows &A, const cgx_opt
   if (!band && !slices) return CGX_SUCCESS;
   reset_host_state(h, o.max_iterations, o.tolerance, false, 0);
   CGX_TRY(push_state(h));
+  CUDA_TRY(cudaEventRecord(h->ev[0], h->stream));
   CUDA_TRY(launch_pcg_setup(h, jacobi));
   CUDA_TRY(band ? launch_solve64(h, jacobi, o.loop, ran) : launch_slices64(h, jacobi, ran));
   return CGX_SUCCESS;
@@ -2277,7 +2279,6 @@ static cgx_status solve_fp64(cgx_handle *h, const cgx_options &o,
   const int loop = want_persist ? CGX_LOOP_GRAPH : o.loop;
   bool ran = false;
   if (want_persist) {
-    CUDA_TRY(cudaEventRecord(h->ev[0], s));
     if (h->format == CGX_FORMAT_ELL)
       CGX_TRY(solve_persistent64(
           h, RowsEll{h->ell_length, h->ell_index, h->ell_data, h->ell_width}, o, jacobi, &ran));

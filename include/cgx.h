@@ -122,7 +122,9 @@ typedef struct cgx_result {
   double true_residual;  /* ||k - A x|| / ||k|| in FP64 if requested, else -1 */
   int converged;         /* residual <= tolerance */
   int outer_iterations;  /* MIXED: refinement steps; 0 otherwise */
-  double solve_ms;       /* device time of the solve (CUDA events) */
+  double solve_ms;       /* device time of the solve (CUDA events); FP64: without
+                            the copy of A that the first solve on new values lays
+                            out; MIXED: with its FP32 copies */
   /* CGX_LOOP_KERNELS only: device time per fused kernel class (ms) and the
    * number of launches of each; zero in the other loop modes:
    * (q = A p | r update, and for the learned path the apply z = G G^T r +
