@@ -310,19 +310,30 @@ def _read_profile(name):
         return None
 
 
-# Algorithmic bytes per row of one inner iteration of the persistent inner
-# solves (persist.cuh), full and for the last iteration of a launch (which
-# stops after its residual test): FP32 vectors 4 bytes, U 16, the factor 8.
-#   split learned: q=Ap 24 | r, d 24 | y=G^T r 16 | z 24 | p 12
-#   split Jacobi:  q=Ap 24 | r, d, <r,Cr> 28 | p = C r + b p 16
-#   fused learned: p, d, q 40 | r, y 24 | z 24
-#   fused Jacobi:  p, d, q 40 | r, z 20
+# Bytes per row of one inner iteration with every vector in memory, full and for the
+# last iteration of a launch: FP32 vectors 4 bytes, U 16, the factor 8. This is what
+# the iteration moves as single kernels, in the phases of the fused form and, for the
+# split one, with d += a p beside r -= a q (or, the second table, beside p).
 PERSIST_BYTES = {(2, True): (100, 48), (2, False): (68, 52),
                  (1, True): (88, 64), (1, False): (60, 60)}
-# The learned split form on grids of at least 3M rows (its L2-prefetch
-# variant) applies d += a p in the direction phase, reading p once.
 PERSIST_DEFER_MIN_ROWS = 3_000_000
 PERSIST_BYTES_DEFERRED = {(2, True): (96, 36)}
+# What the launches move (persist.cuh): the phases of one iteration, the last one of a
+# launch (split: without y, z and the new p; fused: all phases, and d's last update),
+# and the vectors that stay in shared memory, in their order, with the bytes a row and
+# iteration that each saves.
+#   split learned: q=Ap 24 | r 12 | y=G^T r 16 | z 24 | d, p 20
+#   split Jacobi:  q=Ap 24 | r, <r,Cr> 16 | d, p 24
+#   fused learned: p, d, q 40 | r, y 24 | z 24
+#   fused Jacobi:  p, d, q 40 | r, z 20
+LAUNCH_BYTES = {(2, True): (96, 48), (2, False): (64, 52),
+                (1, True): (88, 100), (1, False): (60, 72)}
+LAUNCH_RESIDENT = {(2, True): (("z", 8), ("d", 8), ("q", 8), ("r", 8)),
+                   (2, False): (("r", 12), ("d", 8), ("q", 8), ("C", 8)),
+                   (1, True): (("d", 8), ("C", 4)),
+                   (1, False): (("r", 8), ("d", 8), ("q", 8), ("C", 4))}
+RESIDENT_TILES = 192 // 4  # 192 KB a CTA in tiles of 1024 rows
+TILE_ROWS = 148 * 1024     # a tile of every CTA
 PERSIST_KERNEL = {(2, True): "k_inner_split<learned>", (2, False): "k_inner_split<Jacobi>",
                   (1, True): "k_inner_fused<learned>", (1, False): "k_inner_fused<Jacobi>"}
 
@@ -360,6 +371,28 @@ def persist_roofline(args, results, N, peak, peak_kind):
     per_it = prof.get("dram_bytes_per_iteration") if prof else None
     out["traffic"] = per_it * its / launches if per_it else None
     return out
+
+
+def resident_bytes(key, N):
+    """Bytes a row and iteration that the vectors in shared memory save."""
+    tiles, room, saved = -(-N // TILE_ROWS), RESIDENT_TILES, 0.0
+    for _, per_row in LAUNCH_RESIDENT[key]:
+        n = min(room, tiles)
+        room -= n
+        saved += per_row * min(1.0, n * TILE_ROWS / N)
+    return saved
+
+
+def launch_roofline(roof, results, N, learned):
+    """persist_roofline's line with the bytes that the launches move (LAUNCH_BYTES less
+    what stays in shared memory) in place of those with every vector in memory."""
+    key = (results[-1]["inner_form"], learned)
+    saved = resident_bytes(key, N)
+    full, last = (x - saved for x in LAUNCH_BYTES[key])
+    per_launch = (roof["iterations_per_launch"] * full - (full - last)) * N
+    achieved = per_launch / (roof["launch_us"] * 1e-6) / 1e9
+    return dict(roof, all_in_memory_bytes=roof["algorithmic_bytes"], algorithmic_bytes=per_launch,
+                bytes_per_row_iteration=full, achieved=achieved, frac=achieved / roof["peak"])
 
 
 def plain_persistent(args):
@@ -584,7 +617,7 @@ def our_arm(args, world, rank, local):
     roof = fp64_roof if args.path == "plain" else inner_roof
     persist = persist_roofline(args, results, N, peak, peak_kind)
     if persist is not None:
-        roof = persist
+        roof = launch_roofline(persist, results, N, args.path == "learned")
 
     # End to end through the public C ABI: pinned host inputs uploaded every
     # step (matrix, Jacobi C, right-hand side), the learned set-up and
