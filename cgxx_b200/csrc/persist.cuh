@@ -46,8 +46,9 @@
 // 160^3 DRAM and L2. One CTA per SM (128 registers at 512 threads, 64 at 1024:
 // two rows in flight per thread), one warp that does each barrier's sums, and
 // resident vectors took the iteration (us) from 12.4 to 11.3 (96^3 Jacobi), 21.7
-// to 17.7 (128^3), 45.0 to 38.1 (160^3), and learned 18.2 to 16.4, 41.0 to 32.5
-// and 71.5 to 70.3; 24^3: 7.5 to 4.8 and 9.3 to 6.6.
+// to 17.7 (128^3), 45.0 to 38.1 (160^3), and learned 18.2 to 16.4 and 41.0 to 32.5;
+// 24^3: 7.5 to 4.8 and 9.3 to 6.6. At 160^3 learned they are level (69.1 before, 68.3
+// to 70 now), although DRAM carries 227 MB an iteration instead of 268.
 //
 // Every wait of a cooperative launch is bounded: a CTA that gives up sets
 // kErrGridSync in CgState::error and leaves the loop, so the launch always ends

@@ -37,8 +37,8 @@
 // barriers cost more than those reads.
 //
 // What bounds it: up to 64^3 the barriers (2.0-2.5 us each, gridred.cuh); at
-// 160^3 DRAM (104 bytes per row and iteration, 426 MB, of which L2 serves part:
-// 76 us against 65 at the measured 6.54 TB/s). us per iteration, graph ->
+// 160^3 DRAM (104 bytes per row and iteration, 426 MB, of which DRAM carries 398:
+// 77 us against 61 at the measured 6.54 TB/s). us per iteration, graph ->
 // persistent: 64^2 5-point 17.5 -> 4.6, 257^2 19.3 -> 5.5, 97x64x83 7-point
 // (ELL) 26.6 -> 11.2, 128^3 68.6 -> 36.4, 160^3 138 -> 77, 27-point 96^3 80 ->
 // 43.5.

@@ -77,28 +77,28 @@ typedef enum cgx_precision {
 } cgx_precision;
 
 typedef enum cgx_loop {
-  CGX_LOOP_GRAPH = 0,   /* whole solve = one CUDA graph with a while node,
-                           or, on structured-grid matrices, the persistent
-                           launches below where they measured faster: the
-                           mixed paths' inner solves on the band form, and
-                           plain FP64 solves of matrices with sorted rows and
-                           at most 27 column offsets */
+  CGX_LOOP_GRAPH = 0,   /* the fastest form measured: one persistent launch per
+                           plain FP64 solve and per inner solve of a mixed one,
+                           fused or split (below), where A has a layout for it.
+                           Plain: at most 27 column offsets in sorted rows, mostly
+                           filled; else sorted slices (rows of at most 4095 entries
+                           that pad by at most a quarter). Mixed: the band form (the
+                           7- and 5-point stencils), values by offset or uniform
+                           slices (the 27-point stencils), sorted slices. Other
+                           matrices, and a device without room for the layout: the
+                           whole solve, or inner solve, as one CUDA graph with a
+                           while node */
   CGX_LOOP_CHUNKED = 1, /* graph of a fixed number of iterations, host polls */
   CGX_LOOP_KERNELS = 2, /* one launch per fused kernel, each timed by events */
-  CGX_LOOP_PERSISTENT = 3, /* mixed paths on the band form (the 7- and
-                           5-point stencils, any size): each inner solve is
-                           one cooperative launch whose fused phases (three
-                           per learned iteration, two per Jacobi one) meet at
-                           grid-wide barriers; a plain FP64 solve of a matrix
-                           with sorted rows and at most 27 column offsets is
-                           one such launch too (two phases); other solves run
-                           as GRAPH */
-  CGX_LOOP_PERSISTENT_SPLIT = 4 /* the same launch with one phase per kernel
-                           of the GRAPH iteration (five learned, three
-                           Jacobi or plain FP64) and no value formed twice;
-                           also on SELL-U inner products whose slices are all
-                           uniform (the 27-point stencils), where GRAPH takes
-                           it too */
+  CGX_LOOP_PERSISTENT = 3, /* the fused persistent form: mixed, on the band form,
+                           three phases per learned iteration and two per Jacobi
+                           one, which meet at grid-wide barriers; plain, two
+                           phases, by offset; sorted slices (plain) have the split
+                           form only. Other solves run as the graph */
+  CGX_LOOP_PERSISTENT_SPLIT = 4 /* the split form: one phase per kernel of the
+                           graph's iteration (five learned, three Jacobi or plain
+                           FP64) and no value formed twice; on every layout that
+                           GRAPH has */
 } cgx_loop;
 
 /* Solver settings: the reference's CG_* environment switches
@@ -145,8 +145,8 @@ typedef struct cgx_result {
                             persistent launches on the band form, 3 split
                             persistent launches on SELL-U, values by offset or
                             sorted slices (cgx_loop) */
-  int inner_launches;    /* MIXED, inner_form 1 or 2: persistent launches */
-  double inner_ms;       /* MIXED, inner_form 1 or 2: their device time (CUDA
+  int inner_launches;    /* MIXED, inner_form 1 to 3: persistent launches */
+  double inner_ms;       /* MIXED, inner_form 1 to 3: their device time (CUDA
                             events around each launch) */
 } cgx_result;
 
